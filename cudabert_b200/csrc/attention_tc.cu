@@ -209,7 +209,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const int* __rest
   };
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       Cursor c{};
       c.item = static_cast<int>(blockIdx.x);
       for (cursor_seek(c); c.valid; cursor_next(c)) {
@@ -231,7 +231,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQKV, const int* __rest
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_f16(TQ, TK);
       constexpr uint32_t idesc_o = umma_idesc_f16_bmn(TQ, HD);
       const uint32_t sq = smem_u32(smem + SMEM_Q), sk = smem_u32(smem + SMEM_K), sv = smem_u32(smem + SMEM_V),

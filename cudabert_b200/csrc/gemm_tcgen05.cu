@@ -490,7 +490,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int kblocks = kw.kblocks;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -507,7 +507,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (((FLAGS >= 0) ? FLAGS : flags) & EPI_IN_F16) ? umma_idesc_f16(BM, BN) : umma_idesc_bf16(BM, BN);
       int stage = 0;
       uint32_t phase = 0;
@@ -518,12 +518,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         mbar_wait(tempty_bar + acc, acc_phase ^ 1, abort_flag, err, SITE_TMEM_EMPTY);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ready = mbar_test_wait(full_bar + stage, phase);
         for (int kb = 0; kb < kblocks; ++kb) {
-          mbar_wait(full_bar + stage, phase, abort_flag, err, SITE_FULL);
+          if (!ready) mbar_wait(full_bar + stage, phase, abort_flag, err, SITE_FULL);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * C::STAGE_BYTES);
           const uint64_t da = umma_desc_sw128(sa);
           const uint64_t db = umma_desc_sw128(sa + C::A_BYTES);
+          // look at the next stage before this one's MMAs are issued: the answer is there when they are
+          ready = (stage + 1 == C::STAGES) ? mbar_test_wait(full_bar, phase ^ 1) : mbar_test_wait(full_bar + stage + 1, phase);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // advance 16 elements (32 bytes) along K inside the 128-byte swizzle row
@@ -681,7 +684,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int num_pairs = gridDim.x >> 1;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = pair_id; tile < num_tiles; tile += num_pairs) {
@@ -704,7 +707,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t idesc =
           (((FLAGS >= 0) ? FLAGS : flags) & EPI_IN_F16) ? umma_idesc_f16(2 * BM, BN) : umma_idesc_bf16(2 * BM, BN);
       int stage = 0, wb = 0;
@@ -716,13 +719,16 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         mbar_wait(tempty_bar + acc, acc_phase ^ 1, abort_flag, err, SITE_TMEM_EMPTY);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ready = mbar_test_wait(full_bar + stage, phase);
         for (int kb = 0; kb < kblocks; ++kb) {
-          mbar_wait(full_bar + stage, phase, abort_flag, err, SITE_FULL);
+          if (!ready) mbar_wait(full_bar + stage, phase, abort_flag, err, SITE_FULL);
           if (W8) mbar_wait(wfull_bar + wb, wphase, abort_flag, err, SITE_FULL);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * C::STAGE_BYTES);
           const uint64_t da = umma_desc_sw128(sa);
           const uint64_t db = umma_desc_sw128(W8 ? smem_u32(wbuf + wb * C::B_BYTES) : sa + C::A_BYTES);
+          // look at the next stage before this one's MMAs are issued: the answer is there when they are
+          ready = (stage + 1 == C::STAGES) ? mbar_test_wait(full_bar, phase ^ 1) : mbar_test_wait(full_bar + stage + 1, phase);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
           umma_commit_pair(empty_bar + stage, 3);

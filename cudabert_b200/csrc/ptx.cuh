@@ -90,6 +90,32 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// Non-blocking look at a phase: issued ahead of other work, its latency hides behind that work.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// True in exactly one lane of the (converged) warp.  The single-thread loops that issue TMA copies and
+// tensor-core instructions are entered through this and not through `lane == 0`: those instructions take
+// warp-uniform operands, and under a condition on the lane number the compiler cannot know that one lane is
+// active, so it wraps every one of them in a loop over the active lanes.  Measured on a B200, one thread
+// issuing: tcgen05.commit 67 -> 26 clocks, tcgen05.mma 50 -> 39, and a whole GEMM main loop (one wait, two
+// TMA copies, four MMAs and a commit per 64-column k-block) 547 -> 373 clocks per k-block at 128 x 64 tiles
+// and 554 -> 519 at 128 x 256, where the tensor pipe itself needs 512.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
