@@ -260,6 +260,15 @@ int cudabert_k_gemm_tcgen05(const void* A_dev, long lda, const void* W_dev, int 
   } else if (!cb::make_tmap_16bit_kmajor(&tmW, W_dev, N, K, static_cast<uint64_t>(K) * 2, cb::gemm_w_box_rows(N))) {
     return 2;
   }
+  CUtensorMap tmA32, tmW32;
+  cb::GemmNarrowMaps narrow;
+  if (K % 128 == 0) {
+    if (!cb::make_tmap_16bit_kmajor(&tmA32, A_dev, M, K, static_cast<uint64_t>(lda) * 2, 32) ||
+        !cb::make_narrow_w_map(&tmW32, W_dev, N, K, (flags & cb::EPI_W_FP8) != 0))
+      return 2;
+    narrow.a32 = &tmA32;
+    narrow.w32 = &tmW32;
+  }
   static thread_local DevErr scratch;
   int* err = err_dev;
   if (!err) {
@@ -274,7 +283,7 @@ int cudabert_k_gemm_tcgen05(const void* A_dev, long lda, const void* W_dev, int 
   epi.bias = bias_dev;
   epi.residual = residual_dev;
   epi.colscale = colscale_dev;
-  const int n = cb::gemm_tcgen05(&tmA, &tmW, M, N, K, out_dev, N, epi, err, sms, nullptr, nullptr);
+  const int n = cb::gemm_tcgen05(&tmA, &tmW, M, N, K, out_dev, N, epi, err, sms, nullptr, nullptr, &narrow);
   if (n < 0) return 3;
   if (cudaDeviceSynchronize() != cudaSuccess) return 4;
   int herr = 0;

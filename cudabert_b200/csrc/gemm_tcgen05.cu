@@ -372,8 +372,10 @@ __device__ __forceinline__ void epilogue_tile(uint32_t t_acc, uint8_t* __restric
     __syncwarp();
   };
 
-  // this warp's share of the tile: chunks of 32 columns in [half * BN / 2, (half + 1) * BN / 2)
-  const int c_begin = half * (BN / 64), c_end = c_begin + BN / 64;
+  // this warp's share of the tile: chunks of 32 columns in [half * BN / 2, (half + 1) * BN / 2); a 32-wide tile is
+  // one chunk, which the first half takes
+  constexpr int CHUNKS = BN >= 64 ? BN / 64 : 1;
+  const int c_begin = half * CHUNKS, c_end = (BN >= 64 || half == 0) ? c_begin + CHUNKS : c_begin;
 #pragma unroll
   for (int c = c_begin; c < c_end; ++c) {
     const int col = c * 32;
@@ -827,6 +829,267 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Few rows: single CTAs with narrow tiles (128 x BN, BN = 32, 64 or 128), the weights fetched ahead.
+//
+// A pass of a few hundred rows is a chain of some 90 (BERT-base) to 180 kernels that each do little; its
+// GEMMs are bound by how long ONE tile takes, not by any rate of the whole chip: a CTA pair's
+// 256 x 256 tile costs 519 clocks per 64 columns of K whether its rows exist or not, and a 768-wide output
+// is three of them.  Here the tile is as narrow as the grid allows (thin_width),
+// a stage is 128 columns of K (one wait and one commit per eight MMAs), and the first stages' weights are requested BEFORE griddep_wait: they depend on no predecessor, so with
+// dependent launch they cross HBM while the kernel before is still at work; what does not fit is asked into L2.
+// Only the A tile waits.  Measured from the end of the predecessor to its own end, inside a pass (one B200):
+// BERT-large, 128 rows: QKV 4.4, attention-output 4.4, FFN1 4.4, FFN2 10.0 us; whole pass 1803 -> 1103 us.  BERT-base,
+// 24 rows: 3.6, 3.6, 3.8, 6.7 us, pass 770 -> 487 us; 8 x 128 tokens (U[32,128]): pass 843 -> 636 us.
+// Of the A tile only the 32-row boxes that hold rows below M are loaded; what the other rows of the
+// shared-memory tile hold reaches accumulator rows that are never stored.
+//
+// Every accumulator element is the sum of its K / 16 products-of-16 in ascending K, as in the other
+// variants, and the tensor core's result for an element does not depend on the tile shape around it (checked
+// bit for bit: tests/test_kernels_gpu.py::test_gemm_tile_choice_keeps_every_bit), so the choice between
+// them may go by the row count without a row's result depending on its batch mates.
+//
+// AR: rows the A tile has room for (32 when M <= 32 for the whole launch, else 128); W8 as in the pair
+// kernel: the stage's E4M3 bytes are widened by four converter warps into the stage's W tile, for
+// the first stages also before griddep_wait.
+template <int BN, int AR, bool W8>
+struct ThinCfg {
+  static constexpr int KS = 128;                               // columns of K per stage: two 64-column operand tiles
+  static constexpr int A_HALF = AR * 128, W_HALF = BN * 128;   // bytes of one 64-column tile
+  static constexpr int RAW_BYTES = W8 ? BN * KS : 0;
+  static constexpr int STAGE_BYTES = 2 * A_HALF + 2 * W_HALF + RAW_BYTES;
+  static constexpr int TAIL = AR < 128 ? (128 - AR) * 128 : 0;  // the MMA reads 128 rows from the last A tile's start
+  static constexpr int BAR_BYTES = 320;
+  static constexpr int FIXED = EPI_STAGE_BYTES + BAR_BYTES + 1024 + TAIL;
+  // as deep as shared memory allows, at most eight; eight cover the whole k loop of K <= 1024
+  static constexpr int FIT = (227 * 1024 - FIXED) / STAGE_BYTES;
+  static constexpr int STAGES = FIT < 8 ? FIT : 8;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIXED;
+  static constexpr int THREADS = GEMM_THREADS + (W8 ? CONV_WARPS * 32 : 0);
+  static constexpr int TMEM_COLS = 2 * BN;
+  static_assert(STAGES >= 2, "stage too large");
+};
+
+template <int BN, int AR, int FLAGS, bool W8>
+__global__ void __launch_bounds__(ThinCfg<BN, AR, W8>::THREADS, 1)
+gemm_tcgen05_thin_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA32,
+                         const __grid_constant__ CUtensorMap tmW32, int M, int N, int K, void* __restrict__ out, int ldo,
+                         const float* __restrict__ bias, const float* __restrict__ colscale, int* err,
+                         const int* __restrict__ m_dev) {
+  using C = ThinCfg<BN, AR, W8>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* epi_stage = smem + C::STAGES * C::STAGE_BYTES + C::TAIL;
+  float* sbias = reinterpret_cast<float*>(epi_stage + EPI_WARPS * EPI_WARP_BYTES);
+  float* sscale = sbias + 256;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + EPI_STAGE_BYTES);  // A (and 16-bit W) of a stage have landed
+  uint64_t* empty_bar = full_bar + C::STAGES;
+  uint64_t* raw_bar = empty_bar + C::STAGES;    // W8: the E4M3 bytes of a stage have landed
+  uint64_t* wfull_bar = raw_bar + C::STAGES;    // W8: ... and are converted
+  uint64_t* tfull_bar = wfull_bar + C::STAGES;
+  uint64_t* tempty_bar = tfull_bar + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert((4 * C::STAGES + 4) * 8 + 8 <= C::BAR_BYTES, "barriers");
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(full_bar + s, W8 ? 1 : 2);  // one arrival when A's bytes are announced, one for 16-bit W's
+      mbar_init(empty_bar + s, 1);
+      mbar_init(raw_bar + s, 1);
+      mbar_init(wfull_bar + s, CONV_WARPS);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(tfull_bar + a, 1);
+      mbar_init(tempty_bar + a, EPI_WARPS);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmA32);
+    tma_prefetch_desc(&tmW32);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // The next kernel may be scheduled from here on: it fetches its own weights while this one works, and
+  // touches nothing of ours before its griddep_wait.
+  griddep_launch();
+
+  const int tiles_n = N / BN;
+  const int ks = K / C::KS;                            // stages of a tile
+  const int ahead = ks < C::STAGES ? ks : C::STAGES;   // stages of the first tile whose weights are fetched ahead
+  const int first_n0 = (static_cast<int>(blockIdx.x) % tiles_n) * BN;
+  // live tiles, known once the predecessors (row_layout among them) are done
+  auto live_rows = [&]() { return m_dev ? min(M, __ldg(m_dev)) : M; };
+  auto tiles_of = [&](int m) { return ((m + BM - 1) / BM) * tiles_n; };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      auto load_w = [&](int stage, int k, int n0) {  // the stage's weights
+        uint8_t* sw = smem + stage * C::STAGE_BYTES + 2 * C::A_HALF;
+        if (W8) {
+          mbar_arrive_expect_tx(raw_bar + stage, C::RAW_BYTES);
+#pragma unroll
+          for (int b = 0; b < BN / 32; ++b)
+            tma_load_2d(sw + 2 * C::W_HALF + b * 32 * C::KS, &tmW32, raw_bar + stage, k, n0 + b * 32);
+        } else {
+          mbar_arrive_expect_tx(full_bar + stage, 2 * C::W_HALF);
+#pragma unroll
+          for (int b = 0; b < 2 * (BN / 32); ++b)
+            tma_load_2d(sw + (b & 1) * C::W_HALF + (b >> 1) * 4096, &tmW32, full_bar + stage, k + (b & 1) * 64, n0 + (b >> 1) * 32);
+        }
+      };
+      for (int s = 0; s < ahead; ++s) load_w(s, s * C::KS, first_n0);
+      griddep_wait();
+      const int m = live_rows(), num_tiles = tiles_of(m);
+      int stage = 0, fetched = ahead;
+      uint32_t phase = 0;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+        const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+        const int boxes = min(AR, m - m0 + 31) / 32;  // 32-row boxes of A that hold live rows
+        for (int k = 0; k < K; k += C::KS) {
+          mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, err, SITE_EMPTY);
+          uint8_t* sa = smem + stage * C::STAGE_BYTES;
+          mbar_arrive_expect_tx(full_bar + stage, boxes * 2 * 4096);
+          if (AR == 128 && boxes == 4) {
+            tma_load_2d(sa, &tmA, full_bar + stage, k, m0);
+            tma_load_2d(sa + C::A_HALF, &tmA, full_bar + stage, k + 64, m0);
+          } else {
+            for (int b = 0; b < boxes; ++b) {
+              tma_load_2d(sa + b * 4096, &tmA32, full_bar + stage, k, m0 + b * 32);
+              tma_load_2d(sa + C::A_HALF + b * 4096, &tmA32, full_bar + stage, k + 64, m0 + b * 32);
+            }
+          }
+          if (fetched > 0) --fetched;  // its weights were requested before the wait
+          else load_w(stage, k, n0);
+          if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+      // a CTA without a live tile: its weights must have landed before the shared memory is given back
+      if (static_cast<int>(blockIdx.x) >= num_tiles) {
+        for (int s = 0; s < ahead; ++s) {
+          if (!W8) mbar_arrive(full_bar + s);
+          mbar_wait(W8 ? raw_bar + s : full_bar + s, 0, abort_flag, err, SITE_FULL);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      griddep_wait();
+      const int num_tiles = tiles_of(live_rows());
+      const uint32_t idesc = umma_idesc_f16(BM, BN);
+      int stage = 0;
+      uint32_t phase = 0;
+      int it = 0;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
+        const int acc = it & 1;
+        const uint32_t acc_phase = (it >> 1) & 1;
+        mbar_wait(tempty_bar + acc, acc_phase ^ 1, abort_flag, err, SITE_TMEM_EMPTY);
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        bool ready = mbar_test_wait(full_bar + stage, phase);
+        for (int kb = 0; kb < ks; ++kb) {
+          if (!ready) mbar_wait(full_bar + stage, phase, abort_flag, err, SITE_FULL);
+          if (W8) mbar_wait(wfull_bar + stage, phase, abort_flag, err, SITE_FULL);
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + stage * C::STAGE_BYTES);
+          const uint64_t da = umma_desc_sw128(sa);
+          const uint64_t db = umma_desc_sw128(sa + 2 * C::A_HALF);
+          ready = (stage + 1 == C::STAGES) ? mbar_test_wait(full_bar, phase ^ 1) : mbar_test_wait(full_bar + stage + 1, phase);
+#pragma unroll
+          for (int k = 0; k < C::KS / UMMA_K; ++k)
+            umma_f16(d_tmem, da + (k >> 2) * (C::A_HALF >> 4) + 2 * (k & 3), db + (k >> 2) * (C::W_HALF >> 4) + 2 * (k & 3), idesc,
+                     (kb | k) != 0);
+          umma_commit(empty_bar + stage);
+          if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        }
+        umma_commit(tfull_bar + acc);
+      }
+    }
+  } else if (W8 && warp >= 2 + EPI_WARPS) {
+    // converter warps: 128 E4M3 bytes per row -> two 64-column fp16 tiles in the swizzled layout.  The stage's W
+    // tile is free when its bytes have landed: the producer requested them after the MMAs that read it.
+    const int t = threadIdx.x - (2 + EPI_WARPS) * 32;  // 0 .. 127
+    int stage = 0;
+    uint32_t phase = 0;
+    auto convert = [&]() {
+      mbar_wait(raw_bar + stage, phase, abort_flag, err, SITE_FULL);
+      uint8_t* dst = smem + stage * C::STAGE_BYTES + 2 * C::A_HALF;
+      const uint8_t* src = dst + 2 * C::W_HALF;
+#pragma unroll
+      for (int i = 0; i < C::RAW_BYTES / (CONV_WARPS * 32 * 16); ++i) {
+        const int idx = i * (CONV_WARPS * 32) + t;
+        const int row = idx >> 3, q = idx & 3, half = (idx >> 2) & 1;
+        const uint4 v = *reinterpret_cast<const uint4*>(src + idx * 16);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        uint32_t h[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          h[2 * j] = e4m3x2_to_f16x2(static_cast<uint16_t>(w[j] & 0xffffu));
+          h[2 * j + 1] = e4m3x2_to_f16x2(static_cast<uint16_t>(w[j] >> 16));
+        }
+        uint8_t* drow = dst + half * C::W_HALF + row * 128;
+        *reinterpret_cast<uint4*>(drow + (((2 * q) ^ (row & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(drow + (((2 * q + 1) ^ (row & 7)) << 4)) = make_uint4(h[4], h[5], h[6], h[7]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(wfull_bar + stage);
+      if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+    };
+    for (int s = 0; s < ahead; ++s) convert();
+    griddep_wait();
+    const int num_tiles = tiles_of(live_rows());
+    const int my_tiles = static_cast<int>(blockIdx.x) < num_tiles ? (num_tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
+    for (int n = my_tiles * ks - ahead; n > 0; --n) convert();
+  } else {
+    // the weights of the first tile's later stages: on their way into L2 while the predecessor works
+    if (warp == 2 && elect_one()) {
+      for (int k = ahead * C::KS; k < K; k += C::KS)
+#pragma unroll
+        for (int b = 0; b < (W8 ? 1 : 2) * (BN / 32); ++b)
+          tma_prefetch_l2_2d(&tmW32, W8 ? k : k + (b & 1) * 64, first_n0 + (W8 ? b : b >> 1) * 32);
+    }
+    __syncwarp();
+    griddep_wait();
+    const int m = live_rows(), num_tiles = tiles_of(m);
+    const LnFold no_ln;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
+      const int acc = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      const int n0 = (tile % tiles_n) * BN;
+      const int m0 = (tile / tiles_n) * BM;
+      stage_tile_vectors<BN, FLAGS>(sbias, sscale, FLAGS, bias, colscale, no_ln, n0);
+      mbar_wait(tfull_bar + acc, acc_phase, abort_flag, err, SITE_TMEM_FULL);
+      epilogue_tile<BN, FLAGS>(tmem_base + acc * BN, epi_stage + (warp - 2) * EPI_WARP_BYTES, sbias, sscale, warp,
+                               (warp - 2) >> 2, lane, m0, n0, m, N, K, out, ldo, FLAGS, nullptr, no_ln, 0.f, 1.f);
+      if (lane == 0) mbar_arrive(tempty_bar + acc);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
 // One thread waits, with the pipeline's own bounded wait, on an mbarrier that nobody ever arrives
 // on: the wait gives up after `limit_ns`, records the time-out in `err` exactly as a broken GEMM
 // pipeline would, and the kernel returns.  Used to check the host's handling of that status.
@@ -978,6 +1241,63 @@ int launch_pair(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, in
   }
 }
 
+template <int BN, int AR, int FLAGS>
+int launch_thin_one(const CUtensorMap* tmA, const GemmNarrowMaps& nm, int M, int N, int K, void* out, int ldo,
+                    const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
+  constexpr bool W8 = (FLAGS & EPI_W_FP8) != 0;
+  using C = ThinCfg<BN, AR, W8>;
+  static std::atomic<bool> attr_set[64] = {};  // per device; a repeated set by a racing thread is harmless
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(gemm_tcgen05_thin_kernel<BN, AR, FLAGS, W8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             C::SMEM_BYTES) != cudaSuccess)
+      return -2;
+    if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+  }
+  const int tiles = ((M + BM - 1) / BM) * (N / BN);
+  const int grid = tiles < num_sms ? tiles : num_sms;
+  return launch_pdl(gemm_tcgen05_thin_kernel<BN, AR, FLAGS, W8>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, stream, *tmA,
+                    *nm.a32, *nm.w32, M, N, K, out, ldo, epi.bias, epi.colscale, err_flag, m_dev) == cudaSuccess ? 1 : -3;
+}
+
+template <int FLAGS>
+int launch_thin(int bn, const CUtensorMap* tmA, const GemmNarrowMaps& nm, int M, int N, int K, void* out, int ldo,
+                const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
+  if (bn == 128) return launch_thin_one<128, 128, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+  if (bn == 64) return launch_thin_one<64, 128, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+  if (M <= 32) return launch_thin_one<32, 32, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+  return launch_thin_one<32, 128, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+}
+
+// Tile width of the single-CTA narrow kernel for this product, or 0 for the CTA pairs.  A launch takes about (waves of
+// tiles) x (clocks a tile takes per 64 columns of K): 519 for a pair's 256 x 256 tile (512 of them tensor pipe); for
+// 128 x 128 / 64 / 32 tiles the rate at which an SM takes operands when all of them ask (32 / 24 / 20 KB at some 75 B
+// per clock; 128 x 32 alone is bound by the 39 clocks of issuing an MMA).  FP8 weights add the converter's shared-memory
+// round trip.  M is the padded row count, the most there can be.  Measured, whole passes with one width forced, pairs /
+// 128 / 64 / 32 (us): BERT-large 1 x 128 1805 / 1396 / 1170 / 1103, 4 x 128 1823 / 1484 / 1352 / 1370, 8 x 128 1921 /
+// 1687 / 1591 / 1921, 16 x 128 2212 / 2054 / 2336 / 3027, 32 x 128 3164 / 3706 / 4504 / 5817; with FP8 weights 1 x 24
+// 2079 / 1830 / 1372 / 1156, 8 x 128 2265 / 2384 / 2027 / 2466.
+int thin_width(int flags, int M, int N, int K, int num_sms) {
+  switch (flags) {
+    case F_LIN: case F_FFN1: case F_LIN8: case F_FFN18: case F_LIN8W: case F_FFN18W: break;
+    default: return 0;
+  }
+  if (K % 128 != 0 || N % 128 != 0) return 0;
+  const long pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
+  const long pair_tiles = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * (N / 256);
+  long best = ((pair_tiles + pairs - 1) / pairs) * 519;
+  int width = 0;
+  const bool w8 = (flags & EPI_W_FP8) != 0;
+  const int widths[3] = {128, 64, 32}, clocks[3] = {w8 ? 800 : 430, w8 ? 430 : 330, w8 ? 300 : 290};
+  for (int i = 0; i < 3; ++i) {
+    const long tiles = static_cast<long>((M + BM - 1) / BM) * (N / widths[i]);
+    const long cost = ((tiles + num_sms - 1) / num_sms) * clocks[i];
+    if (cost < best) { best = cost; width = widths[i]; }
+  }
+  return width;
+}
+
 bool pair_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("CUDABERT_GEMM_PAIR");
@@ -1003,10 +1323,11 @@ int gemm_block_n(int N) { return (N % 256 == 0) ? 256 : 128; }
 int gemm_split_block_n(int N) { return (N % 256 == 0 && N > 1024) ? 256 : 128; }
 int gemm_split_w_box_rows(int N) { return 128; }  // half of a pair's 256-row tile, or all of a 128-row one
 
-static bool small_tiles_enabled() {
+// CUDABERT_GEMM_SMALL_TILES=0 keeps every product on the kernel that large ones take (same bits)
+static bool thin_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("CUDABERT_GEMM_SMALL_TILES");
-    return e && e[0] == '1';
+    return !(e && e[0] == '0');
   }();
   return on;
 }
@@ -1015,6 +1336,11 @@ bool gemm_uses_pairs(int N) { return pair_enabled() && (N % 256 == 0); }
 
 // Rows of the W tensor map's box: a CTA of a pair loads half of the 256-row tile.
 int gemm_w_box_rows(int N) { return gemm_uses_pairs(N) ? 128 : gemm_block_n(N); }
+
+bool make_narrow_w_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, bool w_fp8) {
+  return w_fp8 ? make_tmap_u8_kmajor(out, base, rows, cols, 128, 32)
+               : make_tmap_16bit_kmajor(out, base, rows, cols, cols * 2, 32);
+}
 
 bool make_tmap_16bit_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
                            uint64_t row_stride_bytes, uint32_t box_rows) {
@@ -1033,13 +1359,15 @@ bool make_tmap_16bit_kmajor(CUtensorMap* out, const void* base, uint64_t rows, u
   return r == CUDA_SUCCESS;
 }
 
-bool make_tmap_u8_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols) {
+bool make_tmap_u8_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_cols,
+                         uint32_t box_rows) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return false;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || (cols & 15)) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols};
-  const cuuint32_t box[2] = {BK, 128};  // 64 bytes x the 128 rows one CTA of a pair converts per k-block
+  if (box_cols == 0 || (box_cols & 15) || box_cols > 256 || box_rows == 0 || box_rows > 256) return false;
+  const cuuint32_t box[2] = {box_cols, box_rows};
   const CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_NONE;
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -1049,7 +1377,8 @@ bool make_tmap_u8_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint
 }
 
 int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, void* out, int ldo,
-                      const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
+                      const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream,
+                      const GemmNarrowMaps* narrow) {
   if (M <= 0 || N <= 0 || K <= 0 || (N % 128) != 0 || (K % BK) != 0 || (ldo % 8) != 0) return -1;
   if ((epi.flags & EPI_BIAS) && !epi.bias) return -1;
   if ((epi.flags & EPI_RESIDUAL) && !epi.residual) return -1;
@@ -1068,15 +1397,19 @@ int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, i
         (!ln.res_stats || !ln.res_gamma || !ln.res_beta || !(epi.flags & EPI_RESIDUAL) || !(epi.flags & EPI_OUT_F32)))
       return -1;
   }
-  // Few rows: a CTA pair's 256 x 256 tiles are too few to occupy the SMs, and the k loop of one
-  // tile is then the whole run time.  Single CTAs with 128 x 128 tiles have a k loop half as long
-  // and four times as many tiles (BERT-base, 8 x 128 tokens: 0.80 against 0.88 ms per pass; one
-  // sequence of 32 tokens: 0.71 against 0.78 ms).  It is opt-in (CUDABERT_GEMM_SMALL_TILES=1):
-  // the two tile shapes do not round identically, so with it a sequence's result depends, in the
-  // last bits, on how many other rows share its batch, and by default it never does.  The choice
-  // compares (waves of tiles) x (tensor-pipe time of one tile's k loop) for the two shapes and takes
-  // the small tiles only for a clear win.  The pair's W map has 128-row boxes, which is what the
-  // 128 x 128 kernel loads too.
+  // Few rows: narrow single-CTA tiles; the same bits from either kernel (gemm_tcgen05_thin_kernel).
+  if (narrow && narrow->a32 && narrow->w32 && thin_enabled() && gemm_uses_pairs(N)) {
+    const int bn = thin_width(epi.flags, M, N, K, num_sms);
+    switch (bn ? epi.flags : 0) {
+      case F_LIN: return launch_thin<F_LIN>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      case F_FFN1: return launch_thin<F_FFN1>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      case F_LIN8: return launch_thin<F_LIN8>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      case F_FFN18: return launch_thin<F_FFN18>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      case F_LIN8W: return launch_thin<F_LIN8W>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      case F_FFN18W: return launch_thin<F_FFN18W>(bn, tmA, *narrow, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+      default: break;
+    }
+  }
   if (epi.flags & EPI_W_FP8) {
     // E4M3 weight bytes: the CTA-pair kernel with converter warps is the one kernel that reads them
     if (N % 256 != 0 || !(epi.flags & EPI_IN_F16)) return -1;
@@ -1085,15 +1418,6 @@ int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, i
   if (epi.flags & EPI_SPLIT3) {  // tile shape by N alone (gemm_split_block_n)
     if (gemm_split_block_n(N) == 256) return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
     return launch<128>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
-  }
-  if (small_tiles_enabled() && gemm_uses_pairs(N) && gemm_w_box_rows(N) == 128 && !(epi.flags & EPI_LN_SUM)) {
-    const long pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
-    const long tiles_p = static_cast<long>((M + 2 * BM - 1) / (2 * BM)) * (N / 256);
-    const long tiles_s = static_cast<long>((M + BM - 1) / BM) * (N / 128);
-    const long cost_p = ((tiles_p + pairs - 1) / pairs) * 2;  // a 256 x 256 x 16 MMA takes twice a 128 x 128 x 16 one
-    const long cost_s = (tiles_s + num_sms - 1) / num_sms;
-    if (cost_s * 10 <= cost_p * 8)
-      return launch<128>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
   }
   if (gemm_uses_pairs(N)) return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
   if (gemm_block_n(N) == 256) return launch<256>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);

@@ -127,8 +127,16 @@ struct GemmEpilogue {
 // box rows 128 (A) and gemm_w_box_rows(N) (W).
 // m_dev (device int, may be null): the live row count; the kernel then computes rows
 // [0, min(M, *m_dev)) while the launch is sized for M.
+// `narrow` (may be null): the same operands as tensor maps with 32-row boxes, A as by make_tmap_16bit_kmajor and W by
+// make_narrow_w_map; with them, products of few rows may take narrower tiles (same bits).
+struct GemmNarrowMaps {
+  const CUtensorMap* a32 = nullptr;
+  const CUtensorMap* w32 = nullptr;
+};
 int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, void* out, int ldo,
-                      const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream);
+                      const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream,
+                      const GemmNarrowMaps* narrow = nullptr);
+bool make_narrow_w_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, bool w_fp8);
 int gemm_block_n(int N);
 // Launches one thread that runs the pipelines' bounded mbarrier wait on a barrier nobody arrives on,
 // with a limit of `limit_ns` (<= the pipelines' own 2 s): after the limit it sets bit 0 of *err_flag
@@ -147,9 +155,10 @@ int gemm_split_w_box_rows(int N);
 bool make_tmap_16bit_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
                            uint64_t row_stride_bytes, uint32_t box_rows);
 
-// Map over a row-major matrix of bytes [rows, cols] (the E4M3 weights of the FP8 mode), box = 64 bytes x
-// 128 rows, no swizzle.
-bool make_tmap_u8_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols);
+// Map over a row-major matrix of bytes [rows, cols] (the E4M3 weights of the FP8 mode), no swizzle.  The
+// default box is the 64 bytes x 128 rows one CTA of a pair converts per k-block.
+bool make_tmap_u8_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_cols = 64,
+                         uint32_t box_rows = 128);
 
 // ---- fp32 CUDA-core GEMM: out[M, N] = A[M, K] (fp32, row stride lda) x W[K, N] (fp32, the
 // on-disk [in, out] layout).  N % 4 == 0, K % 4 == 0.

@@ -262,11 +262,12 @@ bool Model::finish_dense(DenseWeight* d, int prec) {
   }
   if (prec == PREC_FP8 && !fp8_widened_) {
     if (d->N % 256 != 0) return fail(1, "FP8 mode needs dense widths that are multiples of 256");
-    if (!make_tmap_u8_kmajor(&d->tmap, d->w_fp8, d->N, d->K))
+    if (!make_tmap_u8_kmajor(&d->tmap, d->w_fp8, d->N, d->K) || !make_narrow_w_map(&d->tmap32, d->w_fp8, d->N, d->K, true))
       return fail(2, "cuTensorMapEncodeTiled failed for an FP8 weight matrix");
     return true;
   }
-  if (!make_tmap_16bit_kmajor(&d->tmap, d->w, d->N, d->K, static_cast<uint64_t>(d->K) * 2, gemm_w_box_rows(d->N)))
+  if (!make_tmap_16bit_kmajor(&d->tmap, d->w, d->N, d->K, static_cast<uint64_t>(d->K) * 2, gemm_w_box_rows(d->N)) ||
+      !make_narrow_w_map(&d->tmap32, d->w, d->N, d->K, false))
     return fail(2, "cuTensorMapEncodeTiled failed for a weight matrix");
   return true;
 }
@@ -528,7 +529,11 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
               make_tmap_16bit_kmajor(&tm_x1_, x1a_, rows, H_, static_cast<uint64_t>(H_) * 2, 128) &&
               make_tmap_16bit_kmajor(&tm_ctx_, ctx_, rows, H_, static_cast<uint64_t>(H_) * 2, 128) &&
               make_tmap_16bit_kmajor(&tm_z_, z_, rows, F_, static_cast<uint64_t>(F_) * 2, 128) &&
-              make_tmap_qkv(&tm_qkv_, qkv_, rows, H_);
+              make_tmap_qkv(&tm_qkv_, qkv_, rows, H_) &&
+              make_tmap_16bit_kmajor(&tm_x_32_, xa_, rows, H_, static_cast<uint64_t>(H_) * 2, 32) &&
+              make_tmap_16bit_kmajor(&tm_x1_32_, x1a_, rows, H_, static_cast<uint64_t>(H_) * 2, 32) &&
+              make_tmap_16bit_kmajor(&tm_ctx_32_, ctx_, rows, H_, static_cast<uint64_t>(H_) * 2, 32) &&
+              make_tmap_16bit_kmajor(&tm_z_32_, z_, rows, F_, static_cast<uint64_t>(F_) * 2, 32);
     if (!ok) return fail(2, "cuTensorMapEncodeTiled failed for an activation buffer");
   }
   if (planes) {
@@ -635,7 +640,10 @@ bool Model::dense(const DenseWeight& w, const void* A, const CUtensorMap* tmA, i
     } else {
       epi.flags |= EPI_WSCALE;
     }
-    n = gemm_tcgen05(tmA, &w.tmap, M, w.N, w.K, out, w.N, epi, err_dev_, num_sms_, m_dev_cur_, stream_);
+    GemmNarrowMaps narrow;
+    narrow.a32 = tmA == &tm_x_ ? &tm_x_32_ : tmA == &tm_x1_ ? &tm_x1_32_ : tmA == &tm_ctx_ ? &tm_ctx_32_ : tmA == &tm_z_ ? &tm_z_32_ : nullptr;
+    narrow.w32 = &w.tmap32;
+    n = gemm_tcgen05(tmA, &w.tmap, M, w.N, w.K, out, w.N, epi, err_dev_, num_sms_, m_dev_cur_, stream_, &narrow);
   }
   prof_end(kclass);
   if (n < 0) return fail(2, "GEMM launch rejected (code " + std::to_string(n) + ")");

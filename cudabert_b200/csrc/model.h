@@ -37,6 +37,7 @@ struct DenseWeight {      // one projection
   float* colscale = nullptr; // fp8 mode: [N] de-quantisation scale per output column
   int K = 0, N = 0;
   CUtensorMap tmap;          // bf16 / fp8 modes
+  CUtensorMap tmap32;        // the same with 32-row boxes (GemmNarrowMaps)
 };
 
 struct LayerWeights {
@@ -203,6 +204,7 @@ class Model {
   void *xa_ = nullptr, *x1a_ = nullptr, *ctx_ = nullptr, *qkv_ = nullptr, *z_ = nullptr;
   float *pooled_ = nullptr, *probs_ = nullptr;
   CUtensorMap tm_x_, tm_x1_, tm_ctx_, tm_z_, tm_qkv_;
+  CUtensorMap tm_x_32_, tm_x1_32_, tm_ctx_32_, tm_z_32_;  // the GEMM inputs with 32-row boxes (GemmNarrowMaps)
   void* split_ = nullptr;          // fp32 mode on the tensor cores: the bf16 planes of the current GEMM's input, [tokens, 3 K]
   CUtensorMap tm_splitH_, tm_splitF_;  // ... viewed with K = H and K = F
 

@@ -96,6 +96,38 @@ def test_gemm_tcgen05(pybert, M, N, K, flags):
     assert rel <= tol, "rel err %.3g" % rel
 
 
+@pytest.mark.parametrize("N,K", [(256, 128), (768, 768), (2304, 768), (3072, 768), (768, 3072), (1024, 4096), (4096, 1024)])
+@pytest.mark.parametrize("flags", [ENCODER_LINEAR, ENCODER_LINEAR | EPI_GELU, ENCODER_LINEAR_FP8,
+                                   ENCODER_LINEAR_FP8 | EPI_GELU])
+def test_gemm_tile_choice_keeps_every_bit(pybert, N, K, flags):
+    """Few rows take narrow tiles (128 x 32 / 64 / 128, 32-row boxes of A), many rows the CTA pairs' 256 x 256: a
+    row's result may not depend on how many rows are computed beside it.  20 000 rows, then the first m
+    of them on their own, at the edges of boxes and tiles and across the widths the row count
+    selects: not a bit may differ."""
+    M = 20000
+    g = torch.Generator(device="cuda").manual_seed(N + K + flags)
+    A = (torch.randn(M, K, device="cuda", generator=g) * 0.5).half()
+    W = torch.randn(N, K, device="cuda", generator=g) * 0.05
+    if flags & EPI_W_FP8:  # clamped: beyond E4M3's largest number, 448, the conversion gives NaN, which equals nothing
+        W = (W * 2000.0).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+    else:
+        W = (W.bfloat16().float() * W_CONTAINER_SCALE).half()
+    bias = torch.randn(N, device="cuda", generator=g) * 0.1
+    colscale = ((torch.rand(N, device="cuda", generator=g) + 0.5) / 2000.0).contiguous()
+
+    def run(m):
+        out = torch.full((m + 1, N), float("nan"), device="cuda", dtype=torch.float16)  # one row more than may be written
+        rc = pybert.k_gemm_tcgen05(A.data_ptr(), K, W.data_ptr(), m, N, K, out.data_ptr(), flags, bias.data_ptr(), None,
+                                   colscale.data_ptr(), None)
+        assert rc == 0
+        assert torch.isnan(out[m]).all()
+        return out[:m]
+
+    full = run(M)
+    for m in (1, 31, 32, 33, 64, 96, 97, 127, 128, 129, 200, 257, 700, 1100, 2049, 4000):
+        assert torch.equal(run(m), full[:m]), "m = %d" % m
+
+
 def test_gemm_bf16_strided_rows(pybert):
     """The pooler reads row b*S of the hidden states: A rows with a stride larger than K."""
     B, S, H = 37, 13, 768

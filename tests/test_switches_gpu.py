@@ -114,3 +114,14 @@ def test_fp8_operand_switch_keeps_every_bit(run_with):
     widened = run_with(SWITCH_CHILD_PRECISION="fp8", CUDABERT_FP8_OPERAND="widened")
     for case in BASE_CASES + LARGE_CASES:
         np.testing.assert_array_equal(widened[case], in_kernel[case], err_msg=case)
+
+
+def test_narrow_gemm_tiles_keep_every_bit(run_with):
+    """Products of few rows take narrow single-CTA GEMM tiles with the weights fetched ahead;
+    CUDABERT_GEMM_SMALL_TILES=0 keeps them on the CTA pairs.  The tile around an element does not change
+    how the tensor core sums it: same bits, with bf16 and with FP8 weights."""
+    for precision in ("bf16", "fp8"):
+        narrow = run_with(SWITCH_CHILD_PRECISION=precision)
+        pairs = run_with(SWITCH_CHILD_PRECISION=precision, CUDABERT_GEMM_SMALL_TILES="0")
+        for case in BASE_CASES + LARGE_CASES:
+            np.testing.assert_array_equal(pairs[case], narrow[case], err_msg="%s %s" % (precision, case))
