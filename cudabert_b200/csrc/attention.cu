@@ -528,16 +528,31 @@ attention_f16_persist_kernel(const __grid_constant__ CUtensorMap tmQKV, const in
 }
 
 // ---------------------------------------------------------------- fp32 path
-constexpr int FQ = 32;  // queries per CTA: 8 warps x 4 queries
-constexpr int FK = 32;  // keys per chunk: one per lane
+// A CTA takes 32 queries of one (sequence, head), 8 per warp, and walks the keys in chunks of 32, one per lane.  What
+// bounds it on the CUDA cores is shared-memory reads per multiply-add, so every value read serves several: in Q.K^T
+// a lane's 4 elements of its key (one 16-byte read) meet the same 4 of 8 queries (16-byte broadcasts), in P.V a
+// lane's 2 columns of 4 value rows meet 4 probabilities of each of 8 queries (16-byte broadcasts from the
+// warp's own rows; passing them by shuffle costs an instruction per two multiply-adds).  12 shared-memory
+// passes per 32 multiply-adds either way.  The next chunk's keys and values are on their way (cp.async, two
+// buffers) while this one is worked on.  The order of all sums is that of one query at a time, element by element.
+// Measured on a B200 per layer inside a forward pass, BERT-base, against 8 warps of 4 queries that read a word at a
+// time: 8 x 128 (U[32,128]) 39 -> 22 us, 24 x 101 117 -> 57 us.
+constexpr int FWARPS = 4;
+constexpr int FQW = 8;             // queries per warp
+constexpr int FQ = FWARPS * FQW;   // queries per CTA
+constexpr int FK = 32;             // keys per chunk: one per lane
+constexpr int FKP = HD + 4;        // pitch of a key row: a quarter-warp's 16-byte reads fall on different banks
 
-__global__ void __launch_bounds__(256)
+// VEC: qkv and ctx are 16-byte aligned (the encoder's buffers are); otherwise copies and stores go word by word
+template <bool VEC>
+__global__ void __launch_bounds__(FWARPS * 32)
 attention_f32_kernel(const float* __restrict__ qkv, const int* __restrict__ mask, const int* __restrict__ kv_len,
                      const int* __restrict__ row_start, float* __restrict__ ctx, int S, int heads) {
-  __shared__ float sQ[FQ][HD];
-  __shared__ float sK[FK][HD + 1];
-  __shared__ float sV[FK][HD];
-  __shared__ float sBias[FK];
+  __shared__ __align__(16) float sQ[FQ][HD];
+  __shared__ __align__(16) float sK[2][FK][FKP];
+  __shared__ __align__(16) float sV[2][FK][HD];
+  __shared__ __align__(16) float sP[FWARPS][FQW][FK];
+  __shared__ float sBias[2][FK];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q0 = blockIdx.x * FQ, h = blockIdx.y, b = blockIdx.z;
   const int H = heads * HD, ld = 3 * H;
@@ -552,66 +567,112 @@ attention_f32_kernel(const float* __restrict__ qkv, const int* __restrict__ mask
   const float* base = qkv + static_cast<size_t>(first) * ld + h * HD;
   const int* mrow = mask ? mask + static_cast<size_t>(b) * S : nullptr;
 
-  for (int i = tid; i < FQ * HD; i += 256) {
-    const int r = i / HD, c = i % HD;
-    sQ[r][c] = (q0 + r < nq) ? base[static_cast<size_t>(q0 + r) * ld + c] : 0.f;
-  }
-  float m_run[4], l_run[4], o0[4], o1[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) { m_run[q] = -INFINITY; l_run[q] = 0.f; o0[q] = 0.f; o1[q] = 0.f; }
-
-  for (int k0 = 0; k0 < klen; k0 += FK) {
-    __syncthreads();
-    for (int i = tid; i < FK * HD; i += 256) {
-      const int r = i / HD, c = i % HD;
-      const bool ok = (k0 + r) < klen;
-      sK[r][c] = ok ? base[static_cast<size_t>(k0 + r) * ld + H + c] : 0.f;
-      sV[r][c] = ok ? base[static_cast<size_t>(k0 + r) * ld + 2 * H + c] : 0.f;
+  // 32 rows of 64 floats from row r0 on, zeros from row `limit` on
+  auto copy_rows = [&](float* dst, int pitch, const float* src, int r0, int limit) {
+    if (VEC) {
+      for (int i = tid; i < 32 * (HD / 4); i += FWARPS * 32) {
+        const int r = i / (HD / 4), c = (i % (HD / 4)) * 4;
+        const bool ok = r0 + r < limit;
+        cp_async16(smem_u32(dst + r * pitch + c), src + static_cast<size_t>(ok ? r0 + r : 0) * ld + c, ok);
+      }
+    } else {
+      for (int i = tid; i < 32 * HD; i += FWARPS * 32) {
+        const int r = i / HD, c = i % HD;
+        dst[r * pitch + c] = r0 + r < limit ? src[static_cast<size_t>(r0 + r) * ld + c] : 0.f;
+      }
     }
+  };
+  auto load_chunk = [&](int buf, int k0) {
+    copy_rows(&sK[buf][0][0], FKP, base + H, k0, klen);
+    copy_rows(&sV[buf][0][0], HD, base + 2 * H, k0, klen);
     if (tid < FK) {
       const int key = k0 + tid;
       float v = 0.f;
       if (key >= klen) v = -INFINITY;
       else if (use_mask && mrow[key] == 0) v = -10000.0f;
-      sBias[tid] = v;
+      sBias[buf][tid] = v;
     }
+  };
+  copy_rows(&sQ[0][0], HD, base, q0, nq);
+  load_chunk(0, 0);
+  cp_async_commit();
+
+  float m_run[FQW], l_run[FQW], o0[FQW], o1[FQW];
+#pragma unroll
+  for (int q = 0; q < FQW; ++q) { m_run[q] = -INFINITY; l_run[q] = 0.f; o0[q] = 0.f; o1[q] = 0.f; }
+  const bool work = q0 + warp * FQW < nq;  // some query of this warp exists
+
+  int buf = 0;
+  for (int k0 = 0; k0 < klen; k0 += FK, buf ^= 1) {
+    if (k0 + FK < klen) load_chunk(buf ^ 1, k0 + FK);
+    cp_async_commit();
+    cp_async_wait<1>();  // all but the chunk just requested
     __syncthreads();
+    if (work) {
+      float s[FQW];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float* qr = sQ[warp * 4 + q];
-      float s = 0.f;
-#pragma unroll 16
-      for (int d = 0; d < HD; ++d) s = fmaf(qr[d], sK[lane][d], s);
-      s = s * 0.125f + sBias[lane];
-      float mx = s;
+      for (int q = 0; q < FQW; ++q) s[q] = 0.f;
+#pragma unroll 4
+      for (int d = 0; d < HD; d += 4) {
+        const float4 k = *reinterpret_cast<const float4*>(&sK[buf][lane][d]);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_new = fmaxf(m_run[q], mx);
-      const float alpha = expf(m_run[q] - m_new);
-      const float p = expf(s - m_new);
-      float ps = p;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
-      l_run[q] = l_run[q] * alpha + ps;
-      m_run[q] = m_new;
-      float a0 = o0[q] * alpha, a1 = o1[q] * alpha;
-#pragma unroll
-      for (int j = 0; j < FK; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, p, j);
-        a0 = fmaf(pj, sV[j][lane], a0);
-        a1 = fmaf(pj, sV[j][lane + 32], a1);
+        for (int q = 0; q < FQW; ++q) {
+          const float4 v = *reinterpret_cast<const float4*>(&sQ[warp * FQW + q][d]);
+          s[q] = fmaf(v.x, k.x, s[q]);
+          s[q] = fmaf(v.y, k.y, s[q]);
+          s[q] = fmaf(v.z, k.z, s[q]);
+          s[q] = fmaf(v.w, k.w, s[q]);
+        }
       }
-      o0[q] = a0;
-      o1[q] = a1;
+      const float bias = sBias[buf][lane];
+      __syncwarp();  // the probabilities of the chunk before have been read
+#pragma unroll
+      for (int q = 0; q < FQW; ++q) {
+        s[q] = s[q] * 0.125f + bias;
+        float mx = s[q];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float m_new = fmaxf(m_run[q], mx);
+        const float alpha = expf(m_run[q] - m_new);
+        const float p = expf(s[q] - m_new);
+        float ps = p;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
+        l_run[q] = l_run[q] * alpha + ps;
+        m_run[q] = m_new;
+        o0[q] *= alpha;
+        o1[q] *= alpha;
+        sP[warp][q][lane] = p;
+      }
+      __syncwarp();
+#pragma unroll 2
+      for (int j = 0; j < FK; j += 4) {
+        float2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float2*>(&sV[buf][j + i][2 * lane]);
+#pragma unroll
+        for (int q = 0; q < FQW; ++q) {
+          const float4 p = *reinterpret_cast<const float4*>(&sP[warp][q][j]);
+          o0[q] = fmaf(p.x, v[0].x, o0[q]); o1[q] = fmaf(p.x, v[0].y, o1[q]);
+          o0[q] = fmaf(p.y, v[1].x, o0[q]); o1[q] = fmaf(p.y, v[1].y, o1[q]);
+          o0[q] = fmaf(p.z, v[2].x, o0[q]); o1[q] = fmaf(p.z, v[2].y, o1[q]);
+          o0[q] = fmaf(p.w, v[3].x, o0[q]); o1[q] = fmaf(p.w, v[3].y, o1[q]);
+        }
+      }
     }
+    __syncthreads();  // the buffers are free for the chunk after next
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int row = q0 + warp * 4 + q;
+  for (int q = 0; q < FQW; ++q) {
+    const int row = q0 + warp * FQW + q;
     if (row < nq) {
-      float* dst = ctx + (static_cast<size_t>(first) + row) * H + h * HD;
-      dst[lane] = o0[q] / l_run[q];
-      dst[lane + 32] = o1[q] / l_run[q];
+      float* dst = ctx + (static_cast<size_t>(first) + row) * H + h * HD + 2 * lane;
+      if (VEC) {
+        *reinterpret_cast<float2*>(dst) = make_float2(o0[q] / l_run[q], o1[q] / l_run[q]);
+      } else {
+        dst[0] = o0[q] / l_run[q];
+        dst[1] = o1[q] / l_run[q];
+      }
     }
   }
 }
@@ -783,8 +844,10 @@ int attention_f32(const float* qkv, const int* mask, const int* kv_len, const in
                   int S, int heads, cudaStream_t stream) {
   if (B <= 0 || S <= 0 || heads <= 0 || B > 65535) return -1;
   dim3 grid((S + FQ - 1) / FQ, heads, B);
-  return launch_pdl(attention_f32_kernel, grid, dim3(256), 0, stream, qkv, mask, kv_len, row_start, ctx, S, heads) ==
-                 cudaSuccess ? 1 : -3;
+  // a caller of the single-kernel entry points may pass any pointer; rows are multiples of 256 bytes apart
+  const bool vec = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(ctx)) & 15) == 0;
+  return launch_pdl(vec ? attention_f32_kernel<true> : attention_f32_kernel<false>, grid, dim3(FWARPS * 32), 0, stream, qkv,
+                    mask, kv_len, row_start, ctx, S, heads) == cudaSuccess ? 1 : -3;
 }
 
 int row_layout(const int* mask, int* kv_len, int* row_start, int* sched, int B, int S, cudaStream_t stream) {
