@@ -419,23 +419,6 @@ __device__ __forceinline__ void stage_tile_vectors(float* __restrict__ sbias, fl
   asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
 }
 
-// The k-blocks a tile walks.  Plain: K / BK blocks at columns 0, BK, ... of both operands.  EPI_SPLIT3
-// (operands of three bf16 planes of K columns each): six passes over K, one per cross term, the
-// smallest terms first so that the fp32 accumulator keeps them: (A plane, W plane) = (2, 0), (0, 2),
-// (1, 1), (1, 0), (0, 1), (0, 0).
-struct KWalk {
-  int per, kblocks, K;
-  bool split;
-  __device__ KWalk(int K_, bool split_) : per(K_ / BK), kblocks(split_ ? 6 * (K_ / BK) : K_ / BK), K(K_), split(split_) {}
-  __device__ __forceinline__ int col(int kb, uint32_t planes) const {
-    if (!split) return kb * BK;
-    const int pass = kb / per;
-    return static_cast<int>((planes >> (4 * pass)) & 15u) * K + (kb - pass * per) * BK;
-  }
-  __device__ __forceinline__ int a_col(int kb) const { return col(kb, 0x001102u); }
-  __device__ __forceinline__ int w_col(int kb) const { return col(kb, 0x010120u); }
-};
-
 template <int BN, int FLAGS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int M, int N,
@@ -488,8 +471,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int tiles_n = N / BN;
   const int tiles_m = (M + BM - 1) / BM;
   const int num_tiles = tiles_m * tiles_n;
-  const KWalk kw(K, (((FLAGS >= 0) ? FLAGS : flags) & EPI_SPLIT3) != 0);
-  const int kblocks = kw.kblocks;
+  const int kblocks = K / BK;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -502,8 +484,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, err, SITE_EMPTY);
           uint8_t* sa = smem + stage * C::STAGE_BYTES;
           mbar_arrive_expect_tx(full_bar + stage, C::STAGE_BYTES);
-          tma_load_2d(sa, &tmA, full_bar + stage, kw.a_col(kb), m0);
-          tma_load_2d(sa + C::A_BYTES, &tmW, full_bar + stage, kw.w_col(kb), n0);
+          tma_load_2d(sa, &tmA, full_bar + stage, kb * BK, m0);
+          tma_load_2d(sa + C::A_BYTES, &tmW, full_bar + stage, kb * BK, n0);
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -680,8 +662,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int tiles_n = N / BN;
   const int tiles_m = (M + 2 * BM - 1) / (2 * BM);
   const int num_tiles = tiles_m * tiles_n;
-  const KWalk kw(K, !W8 && (((FLAGS >= 0) ? FLAGS : flags) & EPI_SPLIT3) != 0);
-  const int kblocks = kw.kblocks;
+  const int kblocks = K / BK;
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
 
@@ -697,12 +678,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           uint8_t* sa = smem + stage * C::STAGE_BYTES;
           if (leader) mbar_arrive_expect_tx(full_bar + stage, W8 ? 2 * C::A_BYTES : 2 * C::STAGE_BYTES);
           const uint32_t leader_full = mapa_u32(smem_u32(full_bar + stage), 0);
-          tma_load_2d_pair(sa, &tmA, leader_full, kw.a_col(kb), m0);
+          tma_load_2d_pair(sa, &tmA, leader_full, kb * BK, m0);
           if (W8) {  // E4M3 bytes -> the stage's raw buffer; the converter warps take it from there
             mbar_arrive_expect_tx(raw_full_bar + stage, C::RAW_BYTES);
             tma_load_2d(sa + C::A_BYTES, &tmW, raw_full_bar + stage, kb * BK, n0);
           } else {
-            tma_load_2d_pair(sa + C::A_BYTES, &tmW, leader_full, kw.w_col(kb), n0);
+            tma_load_2d_pair(sa + C::A_BYTES, &tmW, leader_full, kb * BK, n0);
           }
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
         }
@@ -1090,6 +1071,255 @@ gemm_tcgen05_thin_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// fp32 product of operands held as three bf16 planes (EPI_SPLIT3, kernels.h): 128 x 128 tiles, a cluster of CS CTAs
+// per tile that share out the k loop.
+//
+// Per 64 columns of K each plane of A and W is loaded ONCE (96 KB) and serves all six cross terms,
+// 24 MMAs of 64 clocks: walking K six times, a plane pair per pass, as one long GEMM loads 192 KB for them
+// and was bound by what it takes to issue and deliver a k-block (0.29 - 0.33 us per pair).  A ring slot is one plane
+// of both operands (32 KB, seven slots), loaded in the order 2, 0, 1; the terms run a2 w0, a0 w2 | a0 w0, a1 w0, a0 w1 |
+// a1 w1, which frees the slots in that order, each as soon as its last term has been issued and completed.
+// a0 w0 accumulates in one set of TMEM columns and the five small terms in another, so the small ones are not
+// rounded against the large sum; they meet in fp32 registers.
+//
+// Split of K (CS): the outputs of the narrow products are few tiles (BERT-base, 657 rows: 36 for N = 768)
+// with a long loop, so CS CTAs take a part of K each and add their fp32 partial tiles through distributed shared
+// memory, in rank order; each CTA finishes some of the columns.  CS goes by N and K alone
+// (split_cluster): a row's bits must not depend on how many rows share its batch.  Shorter chains of
+// tensor-core accumulations also round less: against float64 the errors are smaller than of the six-pass loop
+// (tests/test_kernels_gpu.py::test_gemm_f32_on_tensor_cores prints them).
+// Measured per launch inside a BERT-base pass (one B200), against the six-pass loop: 657 rows QKV 29 -> 18 us,
+// attention-output 22 -> 14, FFN1 29 -> 20, FFN2 67 -> 27.  What bounds it is shared-memory bandwidth: 288 KB per slice of
+// 64 columns (192 read by the MMAs, 96 written by TMA) are 2300 clocks at 128 B per clock, the MMAs 1536.
+struct SplitCfg {
+  static constexpr int SLOTS = 7;
+  static constexpr int TILE_BYTES = BM * BK * 2;       // one plane tile, of A or of W (128 x 64)
+  static constexpr int SLOT_BYTES = 2 * TILE_BYTES;
+  static constexpr int BAR_BYTES = 256;
+  static constexpr int SMEM_BYTES = SLOTS * SLOT_BYTES + BAR_BYTES + 1024;
+  static constexpr int TMEM_COLS = 256;
+  static constexpr int GRANULE = 128 * 128;            // 128 rows x 32 fp32 columns of a partial tile
+};
+
+template <int CS>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int M, int N, int K,
+                   float* __restrict__ out, int ldo, int flags, const float* __restrict__ bias,
+                   const float* __restrict__ residual, int* err, const int* __restrict__ m_dev) {
+  using C = SplitCfg;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::SLOTS * C::SLOT_BYTES);
+  uint64_t* empty_bar = full_bar + C::SLOTS;
+  uint64_t* tfull_bar = empty_bar + C::SLOTS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = CS > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::SLOTS; ++s) {
+      mbar_init(full_bar + s, 2);  // W's bytes announced, A's bytes announced
+      mbar_init(empty_bar + s, 1);
+    }
+    mbar_init(tfull_bar, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmW);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  griddep_launch();
+
+  const int tiles_n = N / 128;
+  const int tile = static_cast<int>(blockIdx.x) / CS;
+  const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * 128;
+  // 64-column slices of this CTA: a share of the k loop, even to within one
+  const int slice0 = K / BK * rank / CS;
+  const int slices = K / BK * (rank + 1) / CS - slice0;
+  const int kbase = slice0 * BK;
+  const int loads = 3 * slices;        // slot uses: three planes per slice, in the order 2, 0, 1
+  auto plane_of = [](int j) { return j == 0 ? 2 : j - 1; };
+  // of the tile's four 32-column chunks, rank r finishes those from first_chunk(r) to first_chunk(r + 1), at most OWN
+  constexpr int OWN = (4 + CS - 1) / CS;
+  auto first_chunk = [](int r) { return (4 * r + CS - 1) / CS; };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      // weights of the first slots, ahead of the wait: they depend on no predecessor
+      const int ahead = loads < C::SLOTS ? loads : C::SLOTS;
+      int j = 0, k = kbase;
+      auto load_w = [&](int slot, int plane, int kk) {
+        mbar_arrive_expect_tx(full_bar + slot, C::TILE_BYTES);
+        tma_load_2d(smem + slot * C::SLOT_BYTES + C::TILE_BYTES, &tmW, full_bar + slot, plane * K + kk, n0);
+      };
+      for (int i = 0; i < ahead; ++i) {
+        load_w(i, plane_of(j), k);
+        if (++j == 3) { j = 0; k += BK; }
+      }
+      griddep_wait();
+      const int m = m_dev ? min(M, __ldg(m_dev)) : M;
+      if (m0 < m) {
+        int slot = 0;
+        uint32_t phase = 0;
+        j = 0; k = kbase;
+        for (int i = 0; i < loads; ++i) {
+          mbar_wait(empty_bar + slot, phase ^ 1, abort_flag, err, SITE_EMPTY);
+          mbar_arrive_expect_tx(full_bar + slot, C::TILE_BYTES);
+          tma_load_2d(smem + slot * C::SLOT_BYTES, &tmA, full_bar + slot, plane_of(j) * K + k, m0);
+          if (i >= ahead) load_w(slot, plane_of(j), k);
+          if (++j == 3) { j = 0; k += BK; }
+          if (++slot == C::SLOTS) { slot = 0; phase ^= 1; }
+        }
+      } else {
+        // no live rows: the weights must have landed before the shared memory is given back
+        for (int i = 0; i < ahead; ++i) {
+          mbar_arrive(full_bar + i);
+          mbar_wait(full_bar + i, 0, abort_flag, err, SITE_FULL);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      griddep_wait();
+      const int m = m_dev ? min(M, __ldg(m_dev)) : M;
+      if (m0 < m) {
+        const uint32_t idesc = umma_idesc_bf16(BM, 128);
+        const uint32_t d_big = tmem_base, d_small = tmem_base + 128;
+        int slot = 0;
+        uint32_t phase = 0;
+        auto next = [&]() { if (++slot == C::SLOTS) { slot = 0; phase ^= 1; } };
+        auto addr = [&](int s) { return smem_u32(smem + s * C::SLOT_BYTES); };
+        auto term = [&](uint32_t d, uint32_t a, uint32_t w, bool first) {
+          const uint64_t da = umma_desc_sw128(a), db = umma_desc_sw128(w + C::TILE_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) umma_f16(d, da + 2 * k, db + 2 * k, idesc, !(first && k == 0));
+        };
+        for (int sl = 0; sl < slices; ++sl) {
+          mbar_wait(full_bar + slot, phase, abort_flag, err, SITE_FULL);
+          const int s2 = slot;
+          next();
+          mbar_wait(full_bar + slot, phase, abort_flag, err, SITE_FULL);
+          const int s0 = slot;
+          next();
+          tc_fence_after();
+          const uint32_t p2 = addr(s2), p0 = addr(s0);
+          term(d_small, p2, p0, sl == 0);
+          term(d_small, p0, p2, false);
+          umma_commit(empty_bar + s2);
+          term(d_big, p0, p0, sl == 0);
+          mbar_wait(full_bar + slot, phase, abort_flag, err, SITE_FULL);
+          const int s1 = slot;
+          next();
+          tc_fence_after();
+          const uint32_t p1 = addr(s1);
+          term(d_small, p1, p0, false);
+          term(d_small, p0, p1, false);
+          umma_commit(empty_bar + s0);
+          term(d_small, p1, p1, false);
+          umma_commit(empty_bar + s1);
+        }
+        umma_commit(tfull_bar);
+      }
+    }
+  } else {
+    griddep_wait();
+  }
+  __syncwarp();
+  griddep_wait();  // every thread: the live row count below is a predecessor's
+  if (m_dev) M = min(M, __ldg(m_dev));
+  const bool live = m0 < M;   // the same in all CTAs of the cluster
+
+  if (live) {
+    const int ew = warp - 2, quarter = warp & 3, half = ew >> 2;
+    if (warp >= 2) {
+      mbar_wait(tfull_bar, 0, abort_flag, err, SITE_TMEM_FULL);
+      tc_fence_after();
+    }
+    __syncwarp();
+    // The partial tiles go where the ring was: it is free once every CTA's MMAs have read their operands.
+    if (CS > 1) cluster_sync_all(); else __syncthreads();
+    // granule [src][g]: CTA src's partial of 128 rows x 32 columns, 16-byte pieces swizzled by the row
+    if (warp >= 2) {
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        const int chunk = half * 2 + cc;  // 32 columns of the tile
+        const int dest = chunk * CS / 4, g = chunk - first_chunk(dest);
+        const int row = quarter * 32 + lane;
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + chunk * 32;
+        uint32_t v[32], u[32];
+        tmem_ld32(t_row, v);
+        tmem_ld32(t_row + 128, u);
+        tmem_ld_wait();
+        uint32_t base = smem_u32(smem) + (rank * OWN + g) * C::GRANULE + row * 128;
+        if (CS > 1) base = mapa_u32(base, dest);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          st_cluster_f4(base + ((q ^ (row & 7)) << 4), __uint_as_float(v[4 * q]) + __uint_as_float(u[4 * q]),
+                        __uint_as_float(v[4 * q + 1]) + __uint_as_float(u[4 * q + 1]),
+                        __uint_as_float(v[4 * q + 2]) + __uint_as_float(u[4 * q + 2]),
+                        __uint_as_float(v[4 * q + 3]) + __uint_as_float(u[4 * q + 3]));
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+    if (CS > 1) cluster_sync_all(); else __syncthreads();
+    if (warp >= 2) {
+      // a warp finishes four rows of a granule at a time: eight lanes cover a row's 32 columns
+      const int c0 = first_chunk(rank), own = first_chunk(rank + 1) - c0;
+      for (int i = ew; i < own * 32; i += EPI_WARPS) {
+        const int g = i >> 5, row = (i & 31) * 4 + (lane >> 3), q = lane & 7;
+        if (m0 + row >= M) continue;
+        const int col = n0 + (c0 + g) * 32 + q * 4;
+        const uint8_t* src = smem + g * C::GRANULE + row * 128 + ((q ^ (row & 7)) << 4);
+        float4 v = *reinterpret_cast<const float4*>(src);
+#pragma unroll
+        for (int r = 1; r < CS; ++r) {
+          const float4 t = *reinterpret_cast<const float4*>(src + r * OWN * C::GRANULE);
+          v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        }
+        if (flags & EPI_BIAS) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(bias + col));
+          v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        }
+        const size_t o = static_cast<size_t>(m0 + row) * ldo + col;
+        if (flags & EPI_RESIDUAL) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(residual + o));
+          v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        }
+        if (flags & EPI_GELU) {
+          gelu_erf2(v.x, v.y);
+          gelu_erf2(v.z, v.w);
+        }
+        if (flags & EPI_TANH) { v.x = tanhf(v.x); v.y = tanhf(v.y); v.z = tanhf(v.z); v.w = tanhf(v.w); }
+        *reinterpret_cast<float4*>(out + o) = v;
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
 // One thread waits, with the pipeline's own bounded wait, on an mbarrier that nobody ever arrives
 // on: the wait gives up after `limit_ns`, records the time-out in `err` exactly as a broken GEMM
 // pipeline would, and the kernel returns.  Used to check the host's handling of that status.
@@ -1134,9 +1364,6 @@ constexpr int F_FFN1_LN = F_FFN1 | EPI_LN_APPLY;   // FFN1 after a folded LayerN
 // attention-output / FFN2 feeding a folded LayerNorm: fp32 sum out (+ fp16 operand, statistics), residual fp32 ...
 constexpr int F_SUM = EPI_BIAS | EPI_IN_F16 | EPI_WSCALE | EPI_OUT_F32 | EPI_RESIDUAL | EPI_LN_SUM;
 constexpr int F_SUM_RLN = F_SUM | EPI_RES_LN;      // ... or itself a folded LayerNorm's output
-constexpr int F_S3 = EPI_BIAS | EPI_OUT_F32 | EPI_SPLIT3;   // fp32 mode on the tensor cores: QKV
-constexpr int F_S3_RES = F_S3 | EPI_RESIDUAL;               // attention-output, FFN2 (+ fp32 residual)
-constexpr int F_S3_FFN1 = F_S3 | EPI_GELU;
 
 template <int BN, int FLAGS>
 int launch_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, void* out, int ldo,
@@ -1161,12 +1388,6 @@ int launch_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int
 template <int BN>
 int launch(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, void* out, int ldo,
            const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
-  switch (epi.flags) {
-    case F_S3_RES:
-      if (BN == 128) return launch_one<128, F_S3_RES>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
-      break;
-    default: break;
-  }
   switch (epi.flags) {
     case F_LIN: return launch_one<BN, F_LIN>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
     case F_FFN1: return launch_one<BN, F_FFN1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
@@ -1232,9 +1453,6 @@ int launch_pair(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, in
     case F_FFN1_LN: return launch_pair_one<F_FFN1_LN>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
     case F_SUM: return launch_pair_one<F_SUM>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
     case F_SUM_RLN: return launch_pair_one<F_SUM_RLN>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    case F_S3: return launch_pair_one<F_S3>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    case F_S3_RES: return launch_pair_one<F_S3_RES>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    case F_S3_FFN1: return launch_pair_one<F_S3_FFN1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
     default:
       if (epi.flags & EPI_W_FP8) return launch_pair_one<-1, true>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
       return launch_pair_one<-1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
@@ -1268,6 +1486,54 @@ int launch_thin(int bn, const CUtensorMap* tmA, const GemmNarrowMaps& nm, int M,
   if (bn == 64) return launch_thin_one<64, 128, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
   if (M <= 32) return launch_thin_one<32, 32, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
   return launch_thin_one<32, 128, FLAGS>(tmA, nm, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+}
+
+// CTAs per tile of the three-plane GEMM, i.e. parts of K, by N and K alone: three for the long loops (FFN2), two for the
+// narrow outputs (attention-output), one where the tiles of a few hundred rows already fill the chip (QKV, FFN1).
+// Three and not four: an SM holds one CTA and a cluster lives in one GPC, so some 32 clusters of four run at once and
+// BERT-base's 36 tiles of FFN2 took two turns (37 us per launch, 657 rows).
+int split_cluster(int N, int K) {
+  const int slices = K / BK;
+  return slices >= 32 ? 3 : (N <= 1024 && slices >= 4) ? 2 : 1;
+}
+
+template <int CS>
+int launch_split_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, float* out, int ldo,
+                     const GemmEpilogue& epi, int* err_flag, const int* m_dev, cudaStream_t stream) {
+  static std::atomic<bool> attr_set[64] = {};  // per device; a repeated set by a racing thread is harmless
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(gemm_split3_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg::SMEM_BYTES) !=
+        cudaSuccess)
+      return -2;
+    if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+  }
+  const long tiles = static_cast<long>((M + BM - 1) / BM) * (N / 128);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * CS));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = SplitCfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, gemm_split3_kernel<CS>, *tmA, *tmW, M, N, K, out, ldo, epi.flags, epi.bias,
+                            static_cast<const float*>(epi.residual), err_flag, m_dev) == cudaSuccess ? 1 : -3;
+}
+
+int launch_split(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, float* out, int ldo,
+                 const GemmEpilogue& epi, int* err_flag, const int* m_dev, cudaStream_t stream) {
+  switch (split_cluster(N, K)) {
+    case 3: return launch_split_one<3>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+    case 2: return launch_split_one<2>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+    default: return launch_split_one<1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+  }
 }
 
 // Tile width of the single-CTA narrow kernel for this product, or 0 for the CTA pairs.  A launch takes about (waves of
@@ -1316,12 +1582,7 @@ int wait_timeout_probe(int* err_flag, unsigned long long limit_ns, cudaStream_t 
 
 int gemm_block_n(int N) { return (N % 256 == 0) ? 256 : 128; }
 
-// Tiles of the three-plane (fp32) GEMM.  Its k loop is six times as long, so with few rows the tiles of
-// a narrow output are few and long: outputs of up to 1024 columns take single CTAs with 128 x 128
-// tiles (four times as many, each half as long as a pair's), wider ones CTA pairs with 256 x 256.  The
-// choice goes by N alone: what a row's result is must not depend on how many rows share its batch.
-int gemm_split_block_n(int N) { return (N % 256 == 0 && N > 1024) ? 256 : 128; }
-int gemm_split_w_box_rows(int N) { return 128; }  // half of a pair's 256-row tile, or all of a 128-row one
+int gemm_split_w_box_rows(int N) { return 128; }
 
 // CUDABERT_GEMM_SMALL_TILES=0 keeps every product on the kernel that large ones take (same bits)
 static bool thin_enabled() {
@@ -1415,9 +1676,9 @@ int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, i
     if (N % 256 != 0 || !(epi.flags & EPI_IN_F16)) return -1;
     return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
   }
-  if (epi.flags & EPI_SPLIT3) {  // tile shape by N alone (gemm_split_block_n)
-    if (gemm_split_block_n(N) == 256) return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    return launch<128>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+  if (epi.flags & EPI_SPLIT3) {
+    if (!(epi.flags & EPI_OUT_F32) || (epi.flags & (EPI_COLSCALE | EPI_WSCALE))) return -1;
+    return launch_split(tmA, tmW, M, N, K, static_cast<float*>(out), ldo, epi, err_flag, m_dev, stream);
   }
   if (gemm_uses_pairs(N)) return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
   if (gemm_block_n(N) == 256) return launch<256>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);

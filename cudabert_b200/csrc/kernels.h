@@ -146,9 +146,7 @@ int wait_timeout_probe(int* err_flag, unsigned long long limit_ns, cudaStream_t 
 // will pick for this N (128 when CTA pairs each load half of a 256-row tile, else gemm_block_n).
 int gemm_w_box_rows(int N);
 bool gemm_uses_pairs(int N);  // the CTA-pair kernel (256 x 256 tiles) serves this width
-// The same for the W operand of an EPI_SPLIT3 GEMM ([N, 3 K] bf16 planes): CTA pairs with 256 x 256
-// tiles for N > 1024, single CTAs with 128 x 128 tiles otherwise.
-int gemm_split_block_n(int N);
+// The same for the W operand of an EPI_SPLIT3 GEMM ([N, 3 K] bf16 planes; 128 x 128 tiles).
 int gemm_split_w_box_rows(int N);
 // Encode a 2-D tiled map over a row-major matrix of 16-bit elements [rows, cols] with
 // `row_stride_bytes` between rows, box = 64 columns (128 bytes, 128-byte swizzle) x `box_rows` rows.
@@ -243,6 +241,8 @@ int transpose_round_bf16(const float* src, __half* dst, int K, int N, cudaStream
 // computed on the device and written to *scale_out.
 int quantize_fp8_weight(const float* src, uint8_t* dst_q, __half* dst_wide, float* scale_out, int K, int N,
                         cudaStream_t stream);
+// dst[i] = the fp16 number of the E4M3 byte src[i] (exact); n % 16 == 0, both 16-byte aligned
+int widen_e4m3(const uint8_t* src, __half* dst, size_t n, cudaStream_t stream);
 int fill_f32(float* dst, float value, size_t n, cudaStream_t stream);
 // LnFold's vectors for the GEMM with bf16-mode weights w ([N, K], fp16 container) that follows a LayerNorm
 // with gamma, beta: c = gamma W, d = beta W + bias.

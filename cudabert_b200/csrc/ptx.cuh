@@ -152,6 +152,11 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t smem_addr, uint32_t rank) 
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+// 16 bytes to shared memory of a CTA of the cluster (address from mapa_u32, or this CTA's own shared address).
+__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
 // Arrive on an mbarrier of another CTA of the cluster (address from mapa_u32), with the default
 // CTA-scope release.  What these arrivals publish is either nothing in memory (an accumulator in TMEM
 // has been read: tcgen05.wait::ld and a tcgen05 fence come first) or shared-memory writes of the
