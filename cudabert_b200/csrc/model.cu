@@ -17,6 +17,7 @@ namespace cb {
 namespace {
 constexpr int MAX_CLASSES = 32;
 constexpr int MAX_SEQ = 512;
+constexpr int FP8_WIDEN_MIN_ROWS = 1536;  // see Model::dense
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 }  // namespace
@@ -88,8 +89,8 @@ bool Model::init(bool large, int gpu, int max_batch, int max_seq, const std::str
     const char* ll = std::getenv("CUDABERT_LAST_LAYER");
     cls_last_ = !(ll && ll[0] == 'f');
     // CUDABERT_FP8_OPERAND=widened: FP8 mode expands the quantised weights to fp16 once, at load, and
-    // runs the 16-bit GEMM on them (same arithmetic, same results; twice the weight memory, and on
-    // 1024 x 64 batches of BERT-large 25.2 against 28.9 ms per pass).  Default: the GEMM reads the E4M3 bytes.
+    // runs the 16-bit GEMM on them (same arithmetic, same results; twice the weight memory).  Default: the
+    // weights stay E4M3 bytes, widened in the GEMM or, for many rows, one matrix at a time before it (dense()).
     const char* f8 = std::getenv("CUDABERT_FP8_OPERAND");
     fp8_widened_ = f8 && f8[0] == 'w';
     // CUDABERT_FP32_GEMM=cuda: fp32 mode multiplies on the CUDA cores (gemm_f32) instead of splitting
@@ -505,6 +506,8 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
   const size_t o_st2 = ln_fold_ ? slot(ct * (H_ / 128) * 2 * sizeof(float)) : 0;
   const bool planes = !lowp && f32_tensor_;
   const size_t o_split = planes ? slot(ct * F_ * 6) : 0;  // three bf16 planes of the widest GEMM input
+  const bool wide = prec_ == PREC_FP8 && !fp8_widened_;
+  const size_t o_wide = wide ? slot(static_cast<size_t>(F_) * H_ * 2) : 0;  // one matrix of weights, widened
   const size_t o_pool = slot(static_cast<size_t>(cbatch) * H_ * sizeof(float));
   const size_t o_probs = slot(static_cast<size_t>(cbatch) * MAX_CLASSES * sizeof(float));
   if (!check(cudaMalloc(&arena_, off), "cudaMalloc(activation arena)")) return false;
@@ -535,6 +538,15 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
               make_tmap_16bit_kmajor(&tm_ctx_32_, ctx_, rows, H_, static_cast<uint64_t>(H_) * 2, 32) &&
               make_tmap_16bit_kmajor(&tm_z_32_, z_, rows, F_, static_cast<uint64_t>(F_) * 2, 32);
     if (!ok) return fail(2, "cuTensorMapEncodeTiled failed for an activation buffer");
+  }
+  if (wide) {
+    wide_ = reinterpret_cast<__half*>(base + o_wide);
+    const int shapes[4][2] = {{3 * H_, H_}, {H_, H_}, {F_, H_}, {H_, F_}};  // N, K
+    for (int i = 0; i < 4; ++i)
+      if (!make_tmap_16bit_kmajor(&tm_wide_[i], wide_, shapes[i][0], shapes[i][1], static_cast<uint64_t>(shapes[i][1]) * 2,
+                                  gemm_w_box_rows(shapes[i][0])) ||
+          !make_narrow_w_map(&tm_wide32_[i], wide_, shapes[i][0], shapes[i][1], false))
+        return fail(2, "cuTensorMapEncodeTiled failed for the widened weights");
   }
   if (planes) {
     split_ = base + o_split;
@@ -634,16 +646,37 @@ bool Model::dense(const DenseWeight& w, const void* A, const CUtensorMap* tmA, i
     // 16-bit modes: fp16 operands and output; the weights' container scale (bf16 mode) or their
     // FP8 de-quantisation scale comes out in the epilogue
     epi.flags |= EPI_IN_F16 | ((flags & EPI_OUT_F32) ? 0 : EPI_OUT_F16);
+    const CUtensorMap *tmW = &w.tmap, *tmW32 = &w.tmap32;
+    int widened = 0;
     if (prec_ == PREC_FP8) {
-      epi.flags |= EPI_COLSCALE | (fp8_widened_ ? 0 : EPI_W_FP8);
+      epi.flags |= EPI_COLSCALE;
       epi.colscale = w.colscale;
+      if (!fp8_widened_) {
+        // Many rows: the bytes are widened to fp16 into one scratch matrix (it stays in L2) right before the GEMM, which
+        // then runs at the 16-bit kernel's rate instead of converting every tile once per row tile.  Few rows: in the GEMM.
+        // Same bits.  BERT-large, in the GEMM / widened first: 1024 x 64 (U[8,64]) 29.7 / 24.2 ms, 64 x 128 6.59 / 5.64,
+        // 32 x 128 3.84 / 3.21, 16 x 128 2.64 / 2.23; at 8 x 128 the narrow tiles with in-kernel conversion take 1.70.
+        if (M >= FP8_WIDEN_MIN_ROWS && gemm_uses_pairs(w.N)) {
+          widened = widen_e4m3(w.w_fp8, wide_, static_cast<size_t>(w.N) * w.K, stream_);
+          if (widened < 0) {
+            prof_end(kclass);
+            return fail(2, "launch failed");
+          }
+          const int i = w.K == F_ ? 3 : w.N == F_ ? 2 : w.N == H_ ? 1 : 0;
+          tmW = &tm_wide_[i];
+          tmW32 = &tm_wide32_[i];
+        } else {
+          epi.flags |= EPI_W_FP8;
+        }
+      }
     } else {
       epi.flags |= EPI_WSCALE;
     }
     GemmNarrowMaps narrow;
     narrow.a32 = tmA == &tm_x_ ? &tm_x_32_ : tmA == &tm_x1_ ? &tm_x1_32_ : tmA == &tm_ctx_ ? &tm_ctx_32_ : tmA == &tm_z_ ? &tm_z_32_ : nullptr;
-    narrow.w32 = &w.tmap32;
-    n = gemm_tcgen05(tmA, &w.tmap, M, w.N, w.K, out, w.N, epi, err_dev_, num_sms_, m_dev_cur_, stream_, &narrow);
+    narrow.w32 = tmW32;
+    n = gemm_tcgen05(tmA, tmW, M, w.N, w.K, out, w.N, epi, err_dev_, num_sms_, m_dev_cur_, stream_, &narrow);
+    if (n > 0) n += widened;
   }
   prof_end(kclass);
   if (n < 0) return fail(2, "GEMM launch rejected (code " + std::to_string(n) + ")");

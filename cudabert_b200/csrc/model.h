@@ -205,6 +205,8 @@ class Model {
   float *pooled_ = nullptr, *probs_ = nullptr;
   CUtensorMap tm_x_, tm_x1_, tm_ctx_, tm_z_, tm_qkv_;
   CUtensorMap tm_x_32_, tm_x1_32_, tm_ctx_32_, tm_z_32_;  // the GEMM inputs with 32-row boxes (GemmNarrowMaps)
+  __half* wide_ = nullptr;         // FP8 mode: one weight matrix widened to fp16, for passes of many rows
+  CUtensorMap tm_wide_[4], tm_wide32_[4];  // ... as QKV, attention-output, FFN1 and FFN2 weights
   void* split_ = nullptr;          // fp32 mode on the tensor cores: the bf16 planes of the current GEMM's input, [tokens, 3 K]
   CUtensorMap tm_splitH_, tm_splitF_;  // ... viewed with K = H and K = F
 

@@ -369,6 +369,26 @@ __global__ void quantize_fp8_kernel(const float* __restrict__ src, uint8_t* __re
   }
 }
 
+// E4M3 bytes -> fp16, exact; a thread takes 16 bytes
+__global__ void __launch_bounds__(256)
+widen_e4m3_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16) {
+  griddep_wait();
+  griddep_launch();
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n16;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const uint4 v = __ldg(src + i);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t h[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      h[2 * j] = e4m3x2_to_f16x2(static_cast<uint16_t>(w[j] & 0xffffu));
+      h[2 * j + 1] = e4m3x2_to_f16x2(static_cast<uint16_t>(w[j] >> 16));
+    }
+    dst[2 * i] = make_uint4(h[0], h[1], h[2], h[3]);
+    dst[2 * i + 1] = make_uint4(h[4], h[5], h[6], h[7]);
+  }
+}
+
 __global__ void fill_f32_kernel(float* dst, float v, size_t n) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -540,6 +560,13 @@ int quantize_fp8_weight(const float* src, uint8_t* dst_q, __half* dst_wide, floa
   dim3 grid((N + 31) / 32, (K + 31) / 32), block(32, 8);
   quantize_fp8_kernel<<<grid, block, 0, stream>>>(src, dst_q, dst_wide, scale_out, K, N);
   return cudaGetLastError() == cudaSuccess ? 3 : -3;
+}
+
+int widen_e4m3(const uint8_t* src, __half* dst, size_t n, cudaStream_t stream) {
+  if ((n & 15) || (reinterpret_cast<uintptr_t>(src) & 15) || (reinterpret_cast<uintptr_t>(dst) & 15)) return -1;
+  const size_t n16 = n / 16, want = (n16 + 255) / 256, cap = static_cast<size_t>(sm_count()) * 8;
+  return launch_pdl(widen_e4m3_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0, stream,
+                    reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst), n16) == cudaSuccess ? 1 : -3;
 }
 
 int transpose_split_bf16x3(const float* src, __nv_bfloat16* dst, int K, int N, cudaStream_t stream) {
