@@ -547,7 +547,8 @@ constexpr int FKP = HD + 4;        // pitch of a key row: a quarter-warp's 16-by
 template <bool VEC>
 __global__ void __launch_bounds__(FWARPS * 32)
 attention_f32_kernel(const float* __restrict__ qkv, const int* __restrict__ mask, const int* __restrict__ kv_len,
-                     const int* __restrict__ row_start, float* __restrict__ ctx, int S, int heads) {
+                     const int* __restrict__ row_start, float* __restrict__ ctx, int S, int heads,
+                     __nv_bfloat16* __restrict__ planes) {
   __shared__ __align__(16) float sQ[FQ][HD];
   __shared__ __align__(16) float sK[2][FK][FKP];
   __shared__ __align__(16) float sV[2][FK][HD];
@@ -667,7 +668,10 @@ attention_f32_kernel(const float* __restrict__ qkv, const int* __restrict__ mask
     const int row = q0 + warp * FQW + q;
     if (row < nq) {
       float* dst = ctx + (static_cast<size_t>(first) + row) * H + h * HD + 2 * lane;
-      if (VEC) {
+      if (planes) {
+        const float y[2] = {o0[q] / l_run[q], o1[q] / l_run[q]};
+        store_planes<2>(planes + (static_cast<size_t>(first) + row) * 3 * H + h * HD + 2 * lane, H, y);
+      } else if (VEC) {
         *reinterpret_cast<float2*>(dst) = make_float2(o0[q] / l_run[q], o1[q] / l_run[q]);
       } else {
         dst[0] = o0[q] / l_run[q];
@@ -841,13 +845,13 @@ int attention_f16_persist(const CUtensorMap* tm_qkv, const int* mask, const int*
 }
 
 int attention_f32(const float* qkv, const int* mask, const int* kv_len, const int* row_start, float* ctx, int B,
-                  int S, int heads, cudaStream_t stream) {
+                  int S, int heads, cudaStream_t stream, __nv_bfloat16* planes) {
   if (B <= 0 || S <= 0 || heads <= 0 || B > 65535) return -1;
   dim3 grid((S + FQ - 1) / FQ, heads, B);
   // a caller of the single-kernel entry points may pass any pointer; rows are multiples of 256 bytes apart
   const bool vec = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(ctx)) & 15) == 0;
   return launch_pdl(vec ? attention_f32_kernel<true> : attention_f32_kernel<false>, grid, dim3(FWARPS * 32), 0, stream, qkv,
-                    mask, kv_len, row_start, ctx, S, heads) == cudaSuccess ? 1 : -3;
+                    mask, kv_len, row_start, ctx, S, heads, planes) == cudaSuccess ? 1 : -3;
 }
 
 int row_layout(const int* mask, int* kv_len, int* row_start, int* sched, int B, int S, cudaStream_t stream) {

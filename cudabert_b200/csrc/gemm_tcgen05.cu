@@ -1301,7 +1301,12 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           gelu_erf2(v.z, v.w);
         }
         if (flags & EPI_TANH) { v.x = tanhf(v.x); v.y = tanhf(v.y); v.z = tanhf(v.z); v.w = tanhf(v.w); }
-        *reinterpret_cast<float4*>(out + o) = v;
+        if (flags & EPI_OUT_PLANES) {
+          const float y[4] = {v.x, v.y, v.z, v.w};
+          store_planes<4>(reinterpret_cast<__nv_bfloat16*>(out) + static_cast<size_t>(m0 + row) * 3 * N + col, N, y);
+        } else {
+          *reinterpret_cast<float4*>(out + o) = v;
+        }
       }
     }
   }
@@ -1645,6 +1650,7 @@ int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, i
   if ((epi.flags & EPI_RESIDUAL) && !epi.residual) return -1;
   if ((epi.flags & EPI_COLSCALE) && !epi.colscale) return -1;
   if ((epi.flags & EPI_SPLIT3) && (epi.flags & (EPI_IN_F16 | EPI_W_FP8))) return -1;  // the planes are bf16
+  if ((epi.flags & EPI_OUT_PLANES) && !(epi.flags & EPI_SPLIT3)) return -1;
   if (epi.flags & (EPI_LN_SUM | EPI_LN_APPLY | EPI_RES_LN)) {  // folded LayerNorm: see LnFold
     const LnFold& ln = epi.ln;
     if (epi.flags & EPI_SPLIT3) return -1;

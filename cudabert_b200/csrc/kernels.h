@@ -73,6 +73,7 @@ enum EpiFlags : int {
                      // side by side (see split_bf16x3); the kernel sums the six leading cross terms over K
   EPI_LN_SUM = 2048,   // this GEMM's output is the input of a LayerNorm that is not run as a kernel (LnFold below)
   EPI_LN_APPLY = 4096, // this GEMM's A operand is such an input, times gamma: normalise in the epilogue
+  EPI_OUT_PLANES = 16384, // EPI_SPLIT3 only: write the result's three bf16 planes [M, 3 N] instead of fp32
   EPI_RES_LN = 8192    // the residual is LayerNorm(residual) of such an input: recompute it
 };
 
@@ -182,7 +183,7 @@ int pooler_f32(const float* x, int rows_per_seq, const int* row_start, const flo
 int attention_f16(const __half* qkv, const int* mask, const int* kv_len, const int* row_start,
                    __half* ctx, int B, int S, int heads, int cls_only, cudaStream_t stream);
 int attention_f32(const float* qkv, const int* mask, const int* kv_len, const int* row_start, float* ctx, int B,
-                  int S, int heads, cudaStream_t stream);
+                  int S, int heads, cudaStream_t stream, __nv_bfloat16* planes = nullptr);
 // tcgen05 variant of attention_f16 (attention_tc.cu): Q, K, V tiles arrive by TMA through `tm_qkv`,
 // a map over the [rows, 3H] projection output made by make_tmap_qkv.  attention_kernel_for says which
 // 16-bit kernel a forward pass of padded length S takes (CUDABERT_ATTENTION=tc|persist|mma forces one).
@@ -210,6 +211,8 @@ int attention_f16_tc(const CUtensorMap* tm_qkv, const int* mask, const int* kv_l
 // of the tile table.
 int row_layout(const int* mask, int* kv_len, int* row_start, int* sched, int B, int S, cudaStream_t stream);
 
+// `planes` (may be null; here, in layernorm, embed_layernorm and, as EPI_OUT_PLANES, in the EPI_SPLIT3 GEMM): the result's three
+// bf16 planes [rows, 3 H], what the next EPI_SPLIT3 GEMM reads; attention and GEMM then write nothing else.
 // ---- row-wise kernels.  The residual stream is kept in fp32; TOut (float or __half) is
 // the copy that feeds the next GEMM.  out_f32 (may be null) receives the same values in fp32.
 // out[row(t)] = LayerNorm(word[ids[t]] + pos[t % S] + type[seg[t]]) for t < tokens = B*S; err bit 1
@@ -218,14 +221,14 @@ int row_layout(const int* mask, int* kv_len, int* row_start, int* sched, int B, 
 template <typename TOut>
 int embed_layernorm(const int* ids, const int* seg, const float* word, const float* pos, const float* type,
                     const float* gamma, const float* beta, TOut* out, float* out_f32, int tokens, int S, int H,
-                    int vocab, int* err_flag, const int* row_start, cudaStream_t stream);
+                    int vocab, int* err_flag, const int* row_start, cudaStream_t stream, __nv_bfloat16* planes = nullptr);
 // out[t] = LayerNorm(x[t] + residual[t]) * gamma + beta; x is fp32 or fp16 (the tensor-core GEMM's
 // dense output), residual (may be null) is the fp32 residual stream.  Rows t < min(tokens, *rows_dev)
 // (rows_dev: device int, may be null) are processed.
 template <typename TIn, typename TOut>
 int layernorm(const TIn* x, const float* residual, const float* gamma, const float* beta, TOut* out, float* out_f32,
               int tokens, int H, const int* rows_dev, cudaStream_t stream, const int* res_rows = nullptr,
-              int res_stride = 1);
+              int res_stride = 1, __nv_bfloat16* planes = nullptr);
 // dst[B*S, H] (fp32) = packed src rows scattered back to the padded layout, zeros for padding.
 int unpack_rows(const float* src, const int* row_start, float* dst, int tokens, int S, int H, cudaStream_t stream);
 // probs[b, :] = softmax(pooled[b, :] . W[H, C] + bias[C]),  C <= 32

@@ -505,7 +505,7 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
   const size_t o_st1 = ln_fold_ ? slot(ct * (H_ / 128) * 2 * sizeof(float)) : 0;
   const size_t o_st2 = ln_fold_ ? slot(ct * (H_ / 128) * 2 * sizeof(float)) : 0;
   const bool planes = !lowp && f32_tensor_;
-  const size_t o_split = planes ? slot(ct * F_ * 6) : 0;  // three bf16 planes of the widest GEMM input
+  const size_t o_split = planes ? slot(ct * F_ * 6) : 0;  // three bf16 planes of FFN2's input
   const bool wide = prec_ == PREC_FP8 && !fp8_widened_;
   const size_t o_wide = wide ? slot(static_cast<size_t>(F_) * H_ * 2) : 0;  // one matrix of weights, widened
   const size_t o_pool = slot(static_cast<size_t>(cbatch) * H_ * sizeof(float));
@@ -549,10 +549,12 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
         return fail(2, "cuTensorMapEncodeTiled failed for the widened weights");
   }
   if (planes) {
-    split_ = base + o_split;
+    // z (4 F bytes per row) is not written in this mode: its slot holds the planes (6 H) of the H-wide GEMM inputs
+    splitH_ = static_cast<__nv_bfloat16*>(z_);
+    splitF_ = reinterpret_cast<__nv_bfloat16*>(base + o_split);
     const uint64_t rows = ct;
-    if (!make_tmap_16bit_kmajor(&tm_splitH_, split_, rows, 3 * static_cast<uint64_t>(H_), static_cast<uint64_t>(H_) * 6, 128) ||
-        !make_tmap_16bit_kmajor(&tm_splitF_, split_, rows, 3 * static_cast<uint64_t>(F_), static_cast<uint64_t>(F_) * 6, 128))
+    if (!make_tmap_16bit_kmajor(&tm_splitH_, splitH_, rows, 3 * static_cast<uint64_t>(H_), static_cast<uint64_t>(H_) * 6, 128) ||
+        !make_tmap_16bit_kmajor(&tm_splitF_, splitF_, rows, 3 * static_cast<uint64_t>(F_), static_cast<uint64_t>(F_) * 6, 128))
       return fail(2, "cuTensorMapEncodeTiled failed for an activation buffer");
   }
   if (h_in_) cudaFreeHost(h_in_);
@@ -631,14 +633,10 @@ bool Model::dense(const DenseWeight& w, const void* A, const CUtensorMap* tmA, i
   int n;
   prof_begin(kclass);
   if (prec_ == PREC_FP32 && f32_tensor_) {
-    // fp32 on the tensor cores: the input's three bf16 planes, then one GEMM over 6 K (kernels.h)
-    n = split_bf16x3(static_cast<const float*>(A), lda, static_cast<__nv_bfloat16*>(split_), M, w.K, m_dev_cur_, stream_);
-    if (n > 0) {
-      epi.flags |= EPI_OUT_F32 | EPI_SPLIT3;
-      const int g = gemm_tcgen05(w.K == H_ ? &tm_splitH_ : &tm_splitF_, &w.tmap, M, w.N, w.K, out, w.N, epi, err_dev_,
-                                 num_sms_, m_dev_cur_, stream_);
-      n = g < 0 ? g : n + g;
-    }
+    // fp32 on the tensor cores: the input's producer has written its three bf16 planes (kernels.h)
+    epi.flags |= EPI_OUT_F32 | EPI_SPLIT3;
+    n = gemm_tcgen05(w.K == H_ ? &tm_splitH_ : &tm_splitF_, &w.tmap, M, w.N, w.K, out, w.N, epi, err_dev_, num_sms_,
+                     m_dev_cur_, stream_);
   } else if (prec_ == PREC_FP32) {
     n = gemm_f32(static_cast<const float*>(A), lda, static_cast<const float*>(w.w), M, w.N, w.K,
                  static_cast<float*>(out), w.N, epi, m_dev_cur_, stream_);
@@ -792,7 +790,7 @@ bool Model::enqueue_forward(const int* d_ids, const int* d_seg, const int* d_mas
                                                        H_, vocab_rows_, err_dev_, rs, stream_));
   } else {
     CB_LAUNCH(KC_EMBED, embed_layernorm<float>(d_ids, d_seg, word_, pos_, type_, emb_g_, emb_b_, xf_, nullptr, T, S, H_,
-                                               vocab_rows_, err_dev_, rs, stream_));
+                                               vocab_rows_, err_dev_, rs, stream_, splitH_));
   }
   bool compact_out = false;  // the final hidden states hold one row per sequence (rows [0, B))
   // Folded LayerNorms (LnFold): in layers 0 .. L-2 the first LayerNorm, in layers 0 .. L-3 the second one
@@ -888,15 +886,17 @@ bool Model::enqueue_forward(const int* d_ids, const int* d_seg, const int* d_mas
       compact_out = cls != 0;
     } else {
       CB_LAUNCH(KC_ATTENTION, attention_f32(static_cast<const float*>(qkv_), d_mask, kv_len_, rs,
-                                            static_cast<float*>(ctx_), B, S, heads_, stream_));
+                                            static_cast<float*>(ctx_), B, S, heads_, stream_, splitH_));
       // fp32 mode: the GEMM epilogue adds the residual, y = ctx.Wo + bo + x
       if (!dense(w.attn_out, ctx_, nullptr, H_, T, y_, EPI_BIAS | EPI_RESIDUAL, xf_, KC_GEMM_ATTN_OUT)) return false;
       CB_LAUNCH(KC_LAYERNORM, (layernorm<float, float>(static_cast<const float*>(y_), nullptr, w.ln1_g, w.ln1_b, x1f_,
-                                                       nullptr, T, H_, live, stream_)));
-      if (!dense(w.ffn1, x1a_, nullptr, H_, T, z_, EPI_BIAS | EPI_GELU, nullptr, KC_GEMM_FFN1)) return false;
+                                                       nullptr, T, H_, live, stream_, nullptr, 1, splitH_)));
+      if (!dense(w.ffn1, x1a_, nullptr, H_, T, splitF_ ? static_cast<void*>(splitF_) : z_,
+                 EPI_BIAS | EPI_GELU | (splitF_ ? EPI_OUT_PLANES : 0), nullptr, KC_GEMM_FFN1))
+        return false;
       if (!dense(w.ffn2, z_, nullptr, F_, T, y_, EPI_BIAS | EPI_RESIDUAL, x1f_, KC_GEMM_FFN2)) return false;
       CB_LAUNCH(KC_LAYERNORM, (layernorm<float, float>(static_cast<const float*>(y_), nullptr, w.ln2_g, w.ln2_b, xf_,
-                                                       nullptr, T, H_, live, stream_)));
+                                                       nullptr, T, H_, live, stream_, nullptr, 1, splitH_)));
     }
   }
   // pooler: rows b*S of the fp32 final hidden states, tanh(dense) -> fp32 [B, H]

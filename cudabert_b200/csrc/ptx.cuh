@@ -368,4 +368,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// The three bf16 planes of an fp32 number (kernels.h): x = b0 + b1 + b2 to within 2^-24 |x|
+__device__ __forceinline__ void split3(float x, __nv_bfloat16& b0, __nv_bfloat16& b1, __nv_bfloat16& b2) {
+  b0 = __float2bfloat16_rn(x);
+  const float r1 = x - __bfloat162float(b0);  // exact
+  b1 = __float2bfloat16_rn(r1);
+  b2 = __float2bfloat16_rn(r1 - __bfloat162float(b1));
+}
+// ... of NV consecutive numbers, plane p to row[p * K ..]; row 2 NV-byte aligned, K % NV == 0
+template <int NV>
+__device__ __forceinline__ void store_planes(__nv_bfloat16* row, int K, const float (&x)[NV]) {
+  static_assert(NV == 2 || NV == 4, "one 4- or 8-byte store per plane");
+  __align__(8) __nv_bfloat16 p[3][NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) split3(x[j], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (NV == 4) *reinterpret_cast<uint2*>(row + static_cast<size_t>(q) * K) = *reinterpret_cast<const uint2*>(p[q]);
+    else *reinterpret_cast<uint32_t*>(row + static_cast<size_t>(q) * K) = *reinterpret_cast<const uint32_t*>(p[q]);
+  }
+}
+
 }  // namespace cb

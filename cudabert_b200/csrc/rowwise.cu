@@ -49,11 +49,12 @@ __device__ __forceinline__ void store4<__half>(__half* p, const float (&y)[4]) {
   *reinterpret_cast<uint2*>(p) = t;
 }
 
-// gamma_at(i), beta_at(i): the lane's vector i of gamma and beta
+// gamma_at(i), beta_at(i): the lane's vector i of gamma and beta; planes_row (may be null): the result's bf16 planes
 template <typename TOut, typename Gamma, typename Beta>
 __device__ __forceinline__ void normalise_and_store(float (&x)[MAXV][4], int nvec, int lane, int H, Gamma gamma_at,
                                                     Beta beta_at, TOut* __restrict__ out_row,
-                                                    float* __restrict__ out_f32_row) {
+                                                    float* __restrict__ out_f32_row,
+                                                    __nv_bfloat16* __restrict__ planes_row) {
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < MAXV; ++i)
@@ -83,6 +84,7 @@ __device__ __forceinline__ void normalise_and_store(float (&x)[MAXV][4], int nve
       y[3] = g.w * ((x[i][3] - mean) * rstd) + bt.w;
       store4<TOut>(out_row + col, y);
       if (out_f32_row) store4<float>(out_f32_row + col, y);
+      if (planes_row) store_planes<4>(planes_row + col, H, y);
     }
   }
 }
@@ -92,7 +94,8 @@ __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32)
 embed_layernorm_kernel(const int* __restrict__ ids, const int* __restrict__ seg, const float* __restrict__ word,
                        const float* __restrict__ pos, const float* __restrict__ type, const float* __restrict__ gamma,
                        const float* __restrict__ beta, TOut* __restrict__ out, float* __restrict__ out_f32, int tokens,
-                       int S, int H, int vocab, int* err, const int* __restrict__ row_start) {
+                       int S, int H, int vocab, int* err, const int* __restrict__ row_start,
+                       __nv_bfloat16* __restrict__ planes) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
   griddep_wait();
@@ -130,7 +133,8 @@ embed_layernorm_kernel(const int* __restrict__ ids, const int* __restrict__ seg,
   }
   normalise_and_store<TOut>(x, nvec, lane, H, [&](int i) { return __ldg(reinterpret_cast<const float4*>(gamma) + i * 32 + lane); },
                               [&](int i) { return __ldg(reinterpret_cast<const float4*>(beta) + i * 32 + lane); },
-                              out + orow * H, out_f32 ? out_f32 + orow * H : nullptr);
+                              out + orow * H, out_f32 ? out_f32 + orow * H : nullptr,
+                            planes ? planes + orow * 3 * H : nullptr);
 }
 
 template <typename TIn>
@@ -161,7 +165,8 @@ template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32)
 layernorm_kernel(const TIn* __restrict__ in, const float* __restrict__ residual, const float* __restrict__ gamma,
                  const float* __restrict__ beta, TOut* __restrict__ out, float* __restrict__ out_f32, int tokens,
-                 int H, const int* __restrict__ rows_dev, const int* __restrict__ res_rows, int res_stride) {
+                 int H, const int* __restrict__ rows_dev, const int* __restrict__ res_rows, int res_stride,
+                 __nv_bfloat16* __restrict__ planes) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
   const int nvec = H / 128;
@@ -193,7 +198,8 @@ layernorm_kernel(const TIn* __restrict__ in, const float* __restrict__ residual,
     }
   if (t >= rows) return;
   normalise_and_store<TOut>(x, nvec, lane, H, [&](int i) { return g[i]; }, [&](int i) { return bt[i]; },
-                            out + static_cast<size_t>(t) * H, out_f32 ? out_f32 + static_cast<size_t>(t) * H : nullptr);
+                            out + static_cast<size_t>(t) * H, out_f32 ? out_f32 + static_cast<size_t>(t) * H : nullptr,
+                            planes ? planes + static_cast<size_t>(t) * 3 * H : nullptr);
 }
 
 // dst[b, s, :] = src[row_start[b] + s, :] for the rows a sequence has, 0 for its padding.
@@ -254,13 +260,6 @@ __global__ void transpose_round_bf16_kernel(const float* __restrict__ src, __hal
   }
 }
 
-__device__ __forceinline__ void split3(float x, __nv_bfloat16& b0, __nv_bfloat16& b1, __nv_bfloat16& b2) {
-  b0 = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(b0);  // exact
-  b1 = __float2bfloat16_rn(r1);
-  b2 = __float2bfloat16_rn(r1 - __bfloat162float(b1));
-}
-
 // dst[n, p K + k] = bf16 plane p of src[k, n], through a 32x33 shared tile
 __global__ void transpose_split_bf16x3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int K,
                                               int N) {
@@ -298,12 +297,7 @@ split_bf16x3_kernel(const float* __restrict__ src, int lds, __nv_bfloat16* __res
     const int m = static_cast<int>(i / quads), k = static_cast<int>(i % quads) << 2;
     const float4 x = *reinterpret_cast<const float4*>(src + static_cast<size_t>(m) * lds + k);
     const float xs[4] = {x.x, x.y, x.z, x.w};
-    __nv_bfloat16 p[3][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) split3(xs[j], p[0][j], p[1][j], p[2][j]);
-    __nv_bfloat16* row = dst + static_cast<size_t>(m) * 3 * K + k;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(row + q * K) = *reinterpret_cast<const uint2*>(p[q]);
+    store_planes<4>(dst + static_cast<size_t>(m) * 3 * K + k, K, xs);
   }
 }
 
@@ -402,11 +396,11 @@ inline bool ln_shape_ok(int H) { return H > 0 && H % 128 == 0 && H <= 1024; }
 template <typename TOut>
 int embed_layernorm(const int* ids, const int* seg, const float* word, const float* pos, const float* type,
                     const float* gamma, const float* beta, TOut* out, float* out_f32, int tokens, int S, int H,
-                    int vocab, int* err_flag, const int* row_start, cudaStream_t stream) {
+                    int vocab, int* err_flag, const int* row_start, cudaStream_t stream, __nv_bfloat16* planes) {
   if (tokens <= 0 || S <= 0 || !ln_shape_ok(H)) return -1;
   const int blocks = (tokens + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
   return launch_pdl(embed_layernorm_kernel<TOut>, dim3(blocks), dim3(ROWS_PER_BLOCK * 32), 0, stream, ids, seg, word, pos,
-                    type, gamma, beta, out, out_f32, tokens, S, H, vocab, err_flag, row_start) == cudaSuccess ? 1 : -3;
+                    type, gamma, beta, out, out_f32, tokens, S, H, vocab, err_flag, row_start, planes) == cudaSuccess ? 1 : -3;
 }
 
 // Persistent form of layernorm_kernel, the default: a fixed grid (two blocks of eight warps per SM)
@@ -434,7 +428,7 @@ __global__ void __launch_bounds__(LNP_THREADS, LNP_BLOCKS_PER_SM)
 layernorm_persist_kernel(const TIn* __restrict__ in, const float* __restrict__ residual, const float* __restrict__ gamma,
                          const float* __restrict__ beta, TOut* __restrict__ out, float* __restrict__ out_f32,
                          int tokens, int H, const int* __restrict__ rows_dev, const int* __restrict__ res_rows,
-                         int res_stride) {
+                         int res_stride, __nv_bfloat16* __restrict__ planes) {
   typedef typename RawVec<TIn>::type Raw;
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (LNP_THREADS / 32);
@@ -471,7 +465,8 @@ layernorm_persist_kernel(const TIn* __restrict__ in, const float* __restrict__ r
     normalise_and_store<TOut>(x, nvec, lane, H, [&](int i) { return __ldg(reinterpret_cast<const float4*>(gamma) + i * 32 + lane); },
                               [&](int i) { return __ldg(reinterpret_cast<const float4*>(beta) + i * 32 + lane); },
                               out + static_cast<size_t>(t) * H,
-                              out_f32 ? out_f32 + static_cast<size_t>(t) * H : nullptr);
+                              out_f32 ? out_f32 + static_cast<size_t>(t) * H : nullptr,
+                            planes ? planes + static_cast<size_t>(t) * 3 * H : nullptr);
     t = next;
   }
 }
@@ -500,7 +495,8 @@ static int sm_count() {
 
 template <typename TIn, typename TOut>
 int layernorm(const TIn* x, const float* residual, const float* gamma, const float* beta, TOut* out, float* out_f32,
-              int tokens, int H, const int* rows_dev, cudaStream_t stream, const int* res_rows, int res_stride) {
+              int tokens, int H, const int* rows_dev, cudaStream_t stream, const int* res_rows, int res_stride,
+              __nv_bfloat16* planes) {
   if (tokens <= 0 || !ln_shape_ok(H)) return -1;
   // As long as every row finds a warp at once (148 SMs hold well over 4096 warps) a launch is one row's chain of latencies,
   // and the one-row-per-warp kernel with its early loads is the faster one: BERT-large 32 x 128 (4096 rows) 3131 -> 3027 us
@@ -510,27 +506,27 @@ int layernorm(const TIn* x, const float* residual, const float* gamma, const flo
     const int want = (tokens + warps_per_block - 1) / warps_per_block;
     const int cap = sm_count() * LNP_BLOCKS_PER_SM;
     return launch_pdl(layernorm_persist_kernel<TIn, TOut>, dim3(want < cap ? want : cap), dim3(LNP_THREADS), 0, stream, x,
-                      residual, gamma, beta, out, out_f32, tokens, H, rows_dev, res_rows, res_stride) == cudaSuccess
+                      residual, gamma, beta, out, out_f32, tokens, H, rows_dev, res_rows, res_stride, planes) == cudaSuccess
                ? 1 : -3;
   }
   const int blocks = (tokens + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
   return launch_pdl(layernorm_kernel<TIn, TOut>, dim3(blocks), dim3(ROWS_PER_BLOCK * 32), 0, stream, x, residual, gamma,
-                    beta, out, out_f32, tokens, H, rows_dev, res_rows, res_stride) == cudaSuccess ? 1 : -3;
+                    beta, out, out_f32, tokens, H, rows_dev, res_rows, res_stride, planes) == cudaSuccess ? 1 : -3;
 }
 
 template int embed_layernorm<float>(const int*, const int*, const float*, const float*, const float*, const float*,
-                                    const float*, float*, float*, int, int, int, int, int*, const int*, cudaStream_t);
+                                    const float*, float*, float*, int, int, int, int, int*, const int*, cudaStream_t, __nv_bfloat16*);
 template int embed_layernorm<__half>(const int*, const int*, const float*, const float*, const float*,
                                             const float*, const float*, __half*, float*, int, int, int, int,
-                                            int*, const int*, cudaStream_t);
+                                            int*, const int*, cudaStream_t, __nv_bfloat16*);
 template int layernorm<float, float>(const float*, const float*, const float*, const float*, float*, float*, int, int,
-                                     const int*, cudaStream_t, const int*, int);
+                                     const int*, cudaStream_t, const int*, int, __nv_bfloat16*);
 template int layernorm<float, __half>(const float*, const float*, const float*, const float*, __half*,
-                                             float*, int, int, const int*, cudaStream_t, const int*, int);
+                                             float*, int, int, const int*, cudaStream_t, const int*, int, __nv_bfloat16*);
 template int layernorm<__half, float>(const __half*, const float*, const float*, const float*, float*, float*, int, int,
-                                      const int*, cudaStream_t, const int*, int);
+                                      const int*, cudaStream_t, const int*, int, __nv_bfloat16*);
 template int layernorm<__half, __half>(const __half*, const float*, const float*, const float*, __half*,
-                                              float*, int, int, const int*, cudaStream_t, const int*, int);
+                                              float*, int, int, const int*, cudaStream_t, const int*, int, __nv_bfloat16*);
 
 int unpack_rows(const float* src, const int* row_start, float* dst, int tokens, int S, int H, cudaStream_t stream) {
   if (tokens <= 0 || S <= 0 || H % 4 != 0) return -1;
