@@ -1078,7 +1078,7 @@ gemm_tcgen05_thin_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 // Per 64 columns of K each plane of A and W is loaded ONCE (96 KB) and serves all six cross terms,
 // 24 MMAs of 64 clocks: walking K six times, a plane pair per pass, as one long GEMM loads 192 KB for them
 // and was bound by what it takes to issue and deliver a k-block (0.29 - 0.33 us per pair).  A ring slot is one plane
-// of both operands (32 KB, seven slots), loaded in the order 2, 0, 1; the terms run a2 w0, a0 w2 | a0 w0, a1 w0, a0 w1 |
+// of both operands (32 KB, seven slots; three with two CTAs per SM, launch_split_cs), loaded in the order 2, 0, 1; the terms run a2 w0, a0 w2 | a0 w0, a1 w0, a0 w1 |
 // a1 w1, which frees the slots in that order, each as soon as its last term has been issued and completed.
 // a0 w0 accumulates in one set of TMEM columns and the five small terms in another, so the small ones are not
 // rounded against the large sum; they meet in fp32 registers.
@@ -1092,8 +1092,9 @@ gemm_tcgen05_thin_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 // Measured per launch inside a BERT-base pass (one B200), against the six-pass loop: 657 rows QKV 29 -> 18 us,
 // attention-output 22 -> 14, FFN1 29 -> 20, FFN2 67 -> 27.  What bounds it is shared-memory bandwidth: 288 KB per slice of
 // 64 columns (192 read by the MMAs, 96 written by TMA) are 2300 clocks at 128 B per clock, the MMAs 1536.
+template <int SLOTS_>
 struct SplitCfg {
-  static constexpr int SLOTS = 7;
+  static constexpr int SLOTS = SLOTS_;
   static constexpr int TILE_BYTES = BM * BK * 2;       // one plane tile, of A or of W (128 x 64)
   static constexpr int SLOT_BYTES = 2 * TILE_BYTES;
   static constexpr int BAR_BYTES = 256;
@@ -1102,12 +1103,12 @@ struct SplitCfg {
   static constexpr int GRANULE = 128 * 128;            // 128 rows x 32 fp32 columns of a partial tile
 };
 
-template <int CS>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+template <int CS, int SLOTS>
+__global__ void __launch_bounds__(GEMM_THREADS, SLOTS == 3 ? 2 : 1)
 gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int M, int N, int K,
                    float* __restrict__ out, int ldo, int flags, const float* __restrict__ bias,
                    const float* __restrict__ residual, int* err, const int* __restrict__ m_dev) {
-  using C = SplitCfg;
+  using C = SplitCfg<SLOTS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::SLOTS * C::SLOT_BYTES);
@@ -1502,15 +1503,15 @@ int split_cluster(int N, int K) {
   return slices >= 32 ? 3 : (N <= 1024 && slices >= 4) ? 2 : 1;
 }
 
-template <int CS>
+template <int CS, int SLOTS>
 int launch_split_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, float* out, int ldo,
                      const GemmEpilogue& epi, int* err_flag, const int* m_dev, cudaStream_t stream) {
   static std::atomic<bool> attr_set[64] = {};  // per device; a repeated set by a racing thread is harmless
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(gemm_split3_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg::SMEM_BYTES) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_split3_kernel<CS, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SplitCfg<SLOTS>::SMEM_BYTES) != cudaSuccess)
       return -2;
     if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
   }
@@ -1518,7 +1519,7 @@ int launch_split_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * CS));
   cfg.blockDim = dim3(GEMM_THREADS);
-  cfg.dynamicSmemBytes = SplitCfg::SMEM_BYTES;
+  cfg.dynamicSmemBytes = SplitCfg<SLOTS>::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1528,16 +1529,28 @@ int launch_split_one(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_split3_kernel<CS>, *tmA, *tmW, M, N, K, out, ldo, epi.flags, epi.bias,
+  return cudaLaunchKernelEx(&cfg, gemm_split3_kernel<CS, SLOTS>, *tmA, *tmW, M, N, K, out, ldo, epi.flags, epi.bias,
                             static_cast<const float*>(epi.residual), err_flag, m_dev) == cudaSuccess ? 1 : -3;
 }
 
+template <int CS>
+int launch_split_cs(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, float* out, int ldo,
+                    const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
+  // More CTAs than one turn of the SMs holds with room to spare: rings of three slots (one slice), two CTAs per SM, so that
+  // one's start and epilogue run under the other's main loop.  Same arithmetic.  BERT-base passes, seven
+  // slots / three (us, one box): 24 x 101 3726 / 3603; 8 x 128, whose 144 - 192 CTAs fit in about one turn, 1445 / 1985.
+  const long ctas = static_cast<long>((M + BM - 1) / BM) * (N / 128) * CS;
+  if (2 * ctas > 3L * num_sms)
+    return launch_split_one<CS, 3>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+  return launch_split_one<CS, 7>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+}
+
 int launch_split(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, int K, float* out, int ldo,
-                 const GemmEpilogue& epi, int* err_flag, const int* m_dev, cudaStream_t stream) {
+                 const GemmEpilogue& epi, int* err_flag, int num_sms, const int* m_dev, cudaStream_t stream) {
   switch (split_cluster(N, K)) {
-    case 3: return launch_split_one<3>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    case 2: return launch_split_one<2>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
-    default: return launch_split_one<1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
+    case 3: return launch_split_cs<3>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+    case 2: return launch_split_cs<2>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
+    default: return launch_split_cs<1>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
   }
 }
 
@@ -1684,7 +1697,7 @@ int gemm_tcgen05(const CUtensorMap* tmA, const CUtensorMap* tmW, int M, int N, i
   }
   if (epi.flags & EPI_SPLIT3) {
     if (!(epi.flags & EPI_OUT_F32) || (epi.flags & (EPI_COLSCALE | EPI_WSCALE))) return -1;
-    return launch_split(tmA, tmW, M, N, K, static_cast<float*>(out), ldo, epi, err_flag, m_dev, stream);
+    return launch_split(tmA, tmW, M, N, K, static_cast<float*>(out), ldo, epi, err_flag, num_sms, m_dev, stream);
   }
   if (gemm_uses_pairs(N)) return launch_pair(tmA, tmW, M, N, K, out, ldo, epi, err_flag, m_dev, stream);
   if (gemm_block_n(N) == 256) return launch<256>(tmA, tmW, M, N, K, out, ldo, epi, err_flag, num_sms, m_dev, stream);
