@@ -283,6 +283,7 @@ int cudabert_k_gemm_tcgen05(const void* A_dev, long lda, const void* W_dev, int 
   epi.bias = bias_dev;
   epi.residual = residual_dev;
   epi.colscale = colscale_dev;
+  cb::NoPdlScope no_pdl;  // the caller's operands may come from a kernel that has only just been launched
   const int n = cb::gemm_tcgen05(&tmA, &tmW, M, N, K, out_dev, N, epi, err, sms, nullptr, nullptr, &narrow);
   if (n < 0) return 3;
   if (cudaDeviceSynchronize() != cudaSuccess) return 4;
@@ -326,6 +327,7 @@ int cudabert_k_gemm_f32_tensor(const float* A_dev, int lda, const float* W_dev, 
     epi.flags = (flags & (cb::EPI_BIAS | cb::EPI_GELU | cb::EPI_RESIDUAL | cb::EPI_TANH)) | cb::EPI_OUT_F32 | cb::EPI_SPLIT3;
     epi.bias = bias_dev;
     epi.residual = residual_dev;
+    cb::NoPdlScope no_pdl;  // the GEMM may fetch W ahead of its predecessor's end
     if (cb::transpose_split_bf16x3(W_dev, w3, K, N, nullptr) < 0 ||
         cb::split_bf16x3(A_dev, lda, a3, M, K, nullptr, nullptr) < 0 ||
         cb::gemm_tcgen05(&tmA, &tmW, M, N, K, out_dev, N, epi, err, sms, nullptr, nullptr) < 0)

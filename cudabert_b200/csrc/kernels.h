@@ -55,6 +55,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Plain stream order for the launches of a scope: callers whose operands may come from the kernel launched just before.
+struct NoPdlScope {
+  bool before = tl_pdl_allowed;
+  NoPdlScope() { tl_pdl_allowed = false; }
+  ~NoPdlScope() { tl_pdl_allowed = before; }
+};
+
 // Epilogue selection, shared by the tcgen05 and the fp32 GEMM:
 //   out = act( acc * colscale[n] + bias[n] + residual[m, n] )
 enum EpiFlags : int {
@@ -130,6 +137,8 @@ struct GemmEpilogue {
 // [0, min(M, *m_dev)) while the launch is sized for M.
 // `narrow` (may be null): the same operands as tensor maps with 32-row boxes, A as by make_tmap_16bit_kmajor and W by
 // make_narrow_w_map; with them, products of few rows may take narrower tiles (same bits).
+// Under dependent launch those kernels, and the EPI_SPLIT3 one, read W before their predecessor has ended: W must not be
+// written by the kernel launched just before.
 struct GemmNarrowMaps {
   const CUtensorMap* a32 = nullptr;
   const CUtensorMap* w32 = nullptr;

@@ -17,7 +17,7 @@ namespace cb {
 namespace {
 constexpr int MAX_CLASSES = 32;
 constexpr int MAX_SEQ = 512;
-constexpr int FP8_WIDEN_MIN_ROWS = 1536;  // see Model::dense
+constexpr int FP8_WIDEN_MIN_ROWS = 2048;  // see Model::dense
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 }  // namespace
@@ -544,8 +544,7 @@ bool Model::ensure_capacity(int B, int S, bool want_hidden_f32) {
     const int shapes[4][2] = {{3 * H_, H_}, {H_, H_}, {F_, H_}, {H_, F_}};  // N, K
     for (int i = 0; i < 4; ++i)
       if (!make_tmap_16bit_kmajor(&tm_wide_[i], wide_, shapes[i][0], shapes[i][1], static_cast<uint64_t>(shapes[i][1]) * 2,
-                                  gemm_w_box_rows(shapes[i][0])) ||
-          !make_narrow_w_map(&tm_wide32_[i], wide_, shapes[i][0], shapes[i][1], false))
+                                  gemm_w_box_rows(shapes[i][0])))
         return fail(2, "cuTensorMapEncodeTiled failed for the widened weights");
   }
   if (planes) {
@@ -653,16 +652,15 @@ bool Model::dense(const DenseWeight& w, const void* A, const CUtensorMap* tmA, i
         // Many rows: the bytes are widened to fp16 into one scratch matrix (it stays in L2) right before the GEMM, which
         // then runs at the 16-bit kernel's rate instead of converting every tile once per row tile.  Few rows: in the GEMM.
         // Same bits.  BERT-large, in the GEMM / widened first: 1024 x 64 (U[8,64]) 29.7 / 24.2 ms, 64 x 128 6.59 / 5.64,
-        // 32 x 128 3.84 / 3.21, 16 x 128 2.64 / 2.23; at 8 x 128 the narrow tiles with in-kernel conversion take 1.70.
+        // 32 x 128 3.84 / 3.21, 16 x 128 2.64 / 2.41; at 8 x 128 the narrow tiles with in-kernel conversion take 1.70.
         if (M >= FP8_WIDEN_MIN_ROWS && gemm_uses_pairs(w.N)) {
           widened = widen_e4m3(w.w_fp8, wide_, static_cast<size_t>(w.N) * w.K, stream_);
           if (widened < 0) {
             prof_end(kclass);
             return fail(2, "launch failed");
           }
-          const int i = w.K == F_ ? 3 : w.N == F_ ? 2 : w.N == H_ ? 1 : 0;
-          tmW = &tm_wide_[i];
-          tmW32 = &tm_wide32_[i];
+          tmW = &tm_wide_[w.K == F_ ? 3 : w.N == F_ ? 2 : w.N == H_ ? 1 : 0];
+          tmW32 = nullptr;  // the narrow tiles fetch weights ahead of their predecessor's end: not these, it writes them
         } else {
           epi.flags |= EPI_W_FP8;
         }

@@ -206,7 +206,7 @@ class Model {
   CUtensorMap tm_x_, tm_x1_, tm_ctx_, tm_z_, tm_qkv_;
   CUtensorMap tm_x_32_, tm_x1_32_, tm_ctx_32_, tm_z_32_;  // the GEMM inputs with 32-row boxes (GemmNarrowMaps)
   __half* wide_ = nullptr;         // FP8 mode: one weight matrix widened to fp16, for passes of many rows
-  CUtensorMap tm_wide_[4], tm_wide32_[4];  // ... as QKV, attention-output, FFN1 and FFN2 weights
+  CUtensorMap tm_wide_[4];         // ... as QKV, attention-output, FFN1 and FFN2 weights
   // fp32 mode on the tensor cores: the bf16 planes of the GEMM inputs, written by their producers: [tokens, 3 H] (in z's
   // slot) for the hidden states and the context, [tokens, 3 F] for FFN2's input
   __nv_bfloat16 *splitH_ = nullptr, *splitF_ = nullptr;

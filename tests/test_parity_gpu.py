@@ -173,6 +173,21 @@ def test_full_size_properties(models, cfg, wname, precision):
     assert bert_oracle.rel_err(full[:2], ref) <= BF16_REL
 
 
+@pytest.mark.parametrize("batch,seq", [(21, 97), (22, 96), (32, 128), (41, 100)])
+def test_fp8_weights_widened_before_the_gemm_keep_every_bit(models, batch, seq):
+    """FP8 passes of 2048 token slots and more widen each weight matrix into one scratch matrix just before its GEMM;
+    smaller ones convert inside the GEMM, whose narrow tiles fetch weights ahead of their predecessor's
+    end.  The scratch is written by that very predecessor, so no GEMM may read it early.  On both sides of
+    the limit, with and without dependent launch (up to 4096 slots): repeated passes and the first rows on
+    their own give the same bits."""
+    m = models("base_affine", "fp8")
+    ids, seg, mask = synth.make_inputs(batch + seq, batch, seq, "uniform:%d:%d" % (seq // 2, seq))
+    full = m.encode([ids, seg, mask])
+    for _ in range(6):
+        assert np.array_equal(m.encode([ids, seg, mask]), full)
+    assert np.array_equal(m.encode([ids[:2], seg[:2], mask[:2]]), full[:2])
+
+
 @pytest.mark.parametrize("precision", ["bf16", "fp8", "fp32"])
 def test_weight_cache_gives_the_same_model(weight_dirs, tmp_path, monkeypatch, precision):
     """CUDABERT_WEIGHT_CACHE: the first load writes the device-ready weights as one file, the second
