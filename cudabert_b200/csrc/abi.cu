@@ -466,6 +466,7 @@ int cudabert_k_embed_layernorm(int half, const int* ids_dev, const int* seg_dev,
 int cudabert_k_layernorm(int out_f16, int in_f16, const void* x_dev, const float* residual_dev,
                          const float* gamma_dev, const float* beta_dev, void* out_dev, float* out_f32_dev, int tokens,
                          int H) {
+  cb::NoPdlScope no_pdl;  // gamma and beta may come from a kernel that has only just been launched
   int n;
   const __half* xh = static_cast<const __half*>(x_dev);
   const float* xf = static_cast<const float*>(x_dev);

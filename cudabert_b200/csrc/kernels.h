@@ -111,7 +111,7 @@ constexpr float LN_EPS_F = 1e-12f;
 // fp32's exponent range, so nothing needs scaling); what is left is below 2^-24 |x|.  A product of two
 // bf16 numbers is exact in the tensor core's fp32 accumulator, so
 //   a . w = a2 w0 + a0 w2 + a1 w1 + a1 w0 + a0 w1 + a0 w0  (+ terms below 2^-24 |a| |w|, dropped)
-// is a GEMM over 6 K with bf16 operands and fp32 accumulation, the small terms first.
+// is six GEMMs over K with bf16 operands and fp32 accumulation, a0 w0 into one accumulator, the small terms into another.
 
 // The encoder's dense weights are ROUNDED to bf16 (8 significand bits: the weight format of the bf16
 // mode) and HELD as fp16 numbers, multiplied by this power of two so that even the smallest of them
