@@ -1288,9 +1288,11 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           const float4 t = *reinterpret_cast<const float4*>(src + r * OWN * C::GRANULE);
           v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
         }
-        if (flags & EPI_BIAS) {
-          const float4 t = __ldg(reinterpret_cast<const float4*>(bias + col));
-          v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+        if (flags & EPI_BIAS) {  // a float at a time: a caller's bias may lie on any 4-byte boundary
+          v.x += __ldg(bias + col);
+          v.y += __ldg(bias + col + 1);
+          v.z += __ldg(bias + col + 2);
+          v.w += __ldg(bias + col + 3);
         }
         const size_t o = static_cast<size_t>(m0 + row) * ldo + col;
         if (flags & EPI_RESIDUAL) {

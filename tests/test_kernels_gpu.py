@@ -192,6 +192,29 @@ def test_gemm_f32_on_tensor_cores(pybert, M, N, K, flags):
         print("max err %.3g (torch fp32 GEMM: %.3g)" % (err.max().item(), (plain - exact.float()).abs().max().item()))
 
 
+@pytest.mark.parametrize("N,K", [(2304, 768), (768, 768), (768, 3072)])   # one, two, three CTAs per tile
+@pytest.mark.parametrize("M", [5, 2500])                                  # deep and short operand rings
+def test_gemm_f32_on_tensor_cores_takes_any_float_pointer_as_bias(pybert, M, N, K):
+    """The bias is a plain float vector: on a 4-, 8- or 12-byte boundary it gives the bits it gives on a
+    16-byte one."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, device="cuda", generator=g)
+    W = torch.randn(K, N, device="cuda", generator=g) * 0.05
+    room = torch.randn(N + 4, device="cuda", generator=g)
+    bias = room[:N].clone()
+    outs = []
+    for shift in range(4):
+        room[shift:shift + N] = bias
+        out = torch.full((M, N), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        assert pybert.k_gemm_f32_tensor(A.data_ptr(), K, W.data_ptr(), M, N, K, out.data_ptr(), EPI_BIAS,
+                                        room[shift:].data_ptr(), None) == 0
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all()
+    for shift in (1, 2, 3):
+        assert torch.equal(outs[shift], outs[0]), "bias shifted by %d floats" % shift
+
+
 @pytest.mark.parametrize("M,H,K1,N2,gelu", [(300, 768, 768, 3072, 1), (1000, 1024, 4096, 3072, 0), (77, 1024, 1024, 4096, 1),
                                             (2049, 768, 3072, 2304, 0), (1, 256, 64, 128, 0)])
 def test_layernorm_folded_into_its_gemms(pybert, M, H, K1, N2, gelu):
