@@ -14,19 +14,24 @@
 namespace cb {
 
 // Launch `kernel` so that it may start while the previous kernel of the stream is still draining
-// (programmatic dependent launch).  Every kernel launched this way executes griddep_wait() before
-// it reads or writes anything a predecessor produces or still reads; until then it only does work
-// that is private to it (barrier set-up, TMEM allocation, descriptor prefetch).
+// (programmatic dependent launch).  Before its griddep_wait() a kernel launched this way only does work that
+// is private to it (barrier set-up, TMEM allocation, descriptor prefetch) and reads data that no kernel still
+// in flight may write: the narrow and the three-plane GEMM fetch weights, the LayerNorm of few rows gamma and beta,
+// the pooler its weights and bias.  In the model those are constants from load time on (weights that the forward
+// pass itself writes go to kernels that read them after the wait); a caller who cannot vouch for that
+// opens a NoPdlScope.  Everything else is read or written after the wait.
 // Whether launch_pdl asks for programmatic dependent launch.  Measured: it shortens a forward pass
 // of a few thousand tokens (BERT-base, 8 x 128: 0.86 against 0.94 ms) and costs about 1 % on one of
 // 25 600 tokens, so the forward pass switches it per call (`tl_pdl_allowed`); CUDABERT_PDL=0 turns it
-// off everywhere, CUDABERT_PDL=1 on everywhere.
+// off everywhere, CUDABERT_PDL=1 on for every forward pass, but not inside a NoPdlScope.
 inline thread_local bool tl_pdl_allowed = true;
+inline thread_local int tl_plain_order = 0;  // NoPdlScopes open on this thread
 inline bool pdl_enabled() {
   static const int forced = [] {
     const char* e = std::getenv("CUDABERT_PDL");
     return !e || !*e ? -1 : (e[0] == '0' ? 0 : 1);
   }();
+  if (tl_plain_order > 0) return false;
   return forced >= 0 ? forced == 1 : tl_pdl_allowed;
 }
 template <typename... KArgs, typename... Args>
@@ -55,11 +60,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// Plain stream order for the launches of a scope: callers whose operands may come from the kernel launched just before.
+// Plain stream order for the launches of a scope, whatever CUDABERT_PDL says: callers whose operands may come from the
+// kernel launched just before.
 struct NoPdlScope {
-  bool before = tl_pdl_allowed;
-  NoPdlScope() { tl_pdl_allowed = false; }
-  ~NoPdlScope() { tl_pdl_allowed = before; }
+  NoPdlScope() { ++tl_plain_order; }
+  ~NoPdlScope() { --tl_plain_order; }
+  NoPdlScope(const NoPdlScope&) = delete;
+  NoPdlScope& operator=(const NoPdlScope&) = delete;
 };
 
 // Epilogue selection, shared by the tcgen05 and the fp32 GEMM:

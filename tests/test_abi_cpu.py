@@ -2,6 +2,7 @@
 declares, fails cleanly without a device, and the oracle's FP8 helper behaves."""
 import os
 import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -98,3 +99,43 @@ def test_reference_application_import_lines():
         "print('ok')\n")
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
+
+
+PDL_PROBE = r"""
+#include <cstdio>
+#include "kernels.h"
+int main() {
+  using namespace cb;
+  const int outside = pdl_enabled();
+  int once, twice, between, pass;
+  {
+    NoPdlScope a;
+    once = pdl_enabled();
+    {
+      NoPdlScope b;
+      twice = pdl_enabled();
+    }
+    between = pdl_enabled();
+    tl_pdl_allowed = true;   // a forward pass's own preference does not end the scope
+    pass = pdl_enabled();
+  }
+  std::printf("%d %d %d %d %d %d", outside, once, twice, between, pass, static_cast<int>(pdl_enabled()));
+}
+"""
+
+
+def test_plain_order_scope_is_stronger_than_the_pdl_switch(tmp_path):
+    """The single-kernel entry points take operands that the kernel launched just before may have
+    written, and some kernels read weights ahead of their predecessor's end under dependent launch: inside
+    a NoPdlScope no launch may ask for it, not even with CUDABERT_PDL=1."""
+    from cudabert_b200 import build
+    src = tmp_path / "pdl_probe.cu"
+    src.write_text(PDL_PROBE)
+    exe = str(tmp_path / "pdl_probe")
+    subprocess.run([build.nvcc()] + build.NVCC_FLAGS + ["-I", build.CSRC, str(src), "-o", exe], check=True)
+    for switch, outside in ((None, 1), ("0", 0), ("1", 1)):
+        env = {k: v for k, v in os.environ.items() if k != "CUDABERT_PDL"}
+        if switch is not None:
+            env["CUDABERT_PDL"] = switch
+        out = subprocess.run([exe], env=env, check=True, capture_output=True, text=True).stdout
+        assert out.split() == [str(outside), "0", "0", "0", "0", str(outside)], "CUDABERT_PDL=%s: %s" % (switch, out)
