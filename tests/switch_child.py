@@ -14,6 +14,7 @@ for p in (ROOT, os.path.join(ROOT, "tests", "golden")):
 def main():
     out_path, specs = sys.argv[1], sys.argv[2:]          # spec = weight_dir:is_large:case,case,...
     import cases
+    from cudabert_b200 import synth
     from cudabert_b200.config import Engin_Config
     from cudabert_b200.cuda_model import Cuda_BERT
     result = {}
@@ -26,7 +27,11 @@ def main():
         cfg.precision = os.environ.get("SWITCH_CHILD_PRECISION", "bf16")
         model = Cuda_BERT(0, cfg)
         for name in names.split(","):
-            ids, seg, mask = cases.case_inputs(name)
+            if name.startswith("rows_"):                 # rows_BxS: seeded inputs of that shape
+                batch, seq = (int(x) for x in name[len("rows_"):].split("x"))
+                ids, seg, mask = synth.make_inputs(batch * seq, batch, seq, "uniform:%d:%d" % (seq // 2, seq))
+            else:
+                ids, seg, mask = cases.case_inputs(name)
             first = model.encode([ids, seg, mask])
             for _ in range(2):
                 again = model.encode([ids, seg, mask])

@@ -192,6 +192,41 @@ def test_gemm_f32_on_tensor_cores(pybert, M, N, K, flags):
         print("max err %.3g (torch fp32 GEMM: %.3g)" % (err.max().item(), (plain - exact.float()).abs().max().item()))
 
 
+@pytest.mark.parametrize("N,K,ctas", [(2304, 768, 1), (3072, 768, 1), (1024, 128, 1), (768, 768, 2), (1024, 256, 2),
+                                      (768, 3072, 3), (1024, 2048, 3)])
+@pytest.mark.parametrize("flags", [EPI_BIAS | EPI_RESIDUAL, EPI_BIAS | EPI_GELU])
+def test_gemm_f32_on_tensor_cores_rows_do_not_depend_on_the_batch(pybert, N, K, ctas, flags):
+    """How many CTAs (`ctas`) share a tile's k loop goes by N and K; the depth of the operand rings and with it the
+    number of CTAs on an SM goes by the row count as well.  Neither may show in a row's result: a batch a few
+    tiles beyond the change of rings, then its first rows on their own, at the edges of tiles and on both
+    sides of that change: not a bit may differ, and the row after the output stays untouched.  The whole batch is
+    held against float64 (the bound of test_gemm_f32_on_tensor_cores)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per_row_tile = N // 128 * ctas
+    deep = 3 * sms // 2 // per_row_tile * 128    # rows up to which rings are deep: 2 CTAs <= 3 SMs
+    M = deep + 300
+    g = torch.Generator(device="cuda").manual_seed(N + K + flags)
+    A = torch.randn(M, K, device="cuda", generator=g)
+    W = torch.randn(K, N, device="cuda", generator=g) * 0.05
+    bias = torch.randn(N, device="cuda", generator=g) * 0.1
+    resid = torch.randn(M, N, device="cuda", generator=g)
+
+    def run(m):
+        out = torch.full((m + 1, N), float("nan"), device="cuda")
+        assert pybert.k_gemm_f32_tensor(A.data_ptr(), K, W.data_ptr(), m, N, K, out.data_ptr(), flags, bias.data_ptr(),
+                                        resid.data_ptr()) == 0
+        assert torch.isnan(out[m]).all()
+        return out[:m]
+
+    full = run(M)
+    ref = _ref_epilogue((A.double() @ W.double()).float(), flags, bias, resid, None)
+    scale = (A.abs().double() @ W.abs().double()).float()
+    bound = 2e-6 * scale + 2e-7 * ref.abs() + 1e-9 + (5e-5 if flags & EPI_GELU else 0.0)
+    assert ((full - ref).abs() <= bound).all()
+    for m in (1, 31, 127, 128, 129, 657, deep - 1, deep, deep + 1, deep + 129):
+        assert torch.equal(run(m), full[:m]), "m = %d" % m
+
+
 @pytest.mark.parametrize("N,K", [(2304, 768), (768, 768), (768, 3072)])   # one, two, three CTAs per tile
 @pytest.mark.parametrize("M", [5, 2500])                                  # deep and short operand rings
 def test_gemm_f32_on_tensor_cores_takes_any_float_pointer_as_bias(pybert, M, N, K):
@@ -303,6 +338,31 @@ def test_attention(pybert, bf16, B, S, heads, mode):
     err = (got - ref).abs().max().item()
     # 16-bit kernels: probabilities and the output are rounded to fp16 (2^-11 relative, values up to ~4)
     assert err <= (4e-3 if bf16 else 1e-4), "max abs err %.3g" % err
+
+
+@pytest.mark.parametrize("B,S,heads,mode", [(2, 1, 12, "none"), (3, 33, 12, "prefix"), (5, 64, 16, "holes"),
+                                            (2, 200, 12, "zero_row")])
+def test_attention_f32_takes_any_float_pointer(pybert, B, S, heads, mode):
+    """The fp32 kernel copies 16 bytes at a time where both pointers allow it and goes word by word
+    otherwise: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(B + S + heads)
+    H = heads * 64
+    n_in, n_out = B * S * 3 * H, B * S * H
+    qkv = torch.randn(n_in, device="cuda", generator=g)
+    mask = _mask(B, S, mode, g)
+    outs = []
+    for in_shift, out_shift in ((0, 0), (1, 0), (0, 1), (3, 2)):
+        x = torch.zeros(n_in + 4, device="cuda")
+        x[in_shift:in_shift + n_in] = qkv
+        room = torch.full((n_out + 4,), float("nan"), device="cuda")
+        ctx = room[out_shift:]
+        assert pybert.k_attention(0, x[in_shift:].data_ptr(), None if mask is None else mask.data_ptr(), ctx.data_ptr(),
+                                  B, S, heads) == 0
+        assert torch.isnan(room[:out_shift]).all() and torch.isnan(ctx[n_out:]).all()
+        outs.append(ctx[:n_out])
+    assert torch.isfinite(outs[0]).all()
+    for got in outs[1:]:
+        assert torch.equal(got, outs[0])
 
 
 @pytest.mark.parametrize("B,S,heads,mode", [(64, 200, 16, "prefix"), (300, 64, 12, "prefix"), (40, 256, 16, "holes"),
@@ -474,3 +534,37 @@ def test_embed_layernorm_and_layernorm(pybert, bf16, H):
                                   typ.data_ptr(), gamma.data_ptr(), beta.data_ptr(), out.data_ptr(), None, T, S, H,
                                   vocab)
     assert rc == 5
+
+
+@pytest.mark.parametrize("in_f16", [0, 1])
+@pytest.mark.parametrize("out_f16", [0, 1])
+@pytest.mark.parametrize("H", [768, 1024])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_layernorm_of_many_rows(pybert, in_f16, out_f16, H, with_residual):
+    """More than 4096 rows take the persistent look-ahead kernel, fewer the one with a row per warp.  The first
+    must be right (against the oracle's LayerNorm) and leave the row after its output alone, and give a row
+    the bits that the second gives it."""
+    g = torch.Generator(device="cuda").manual_seed(H + 2 * in_f16 + out_f16)
+    most = 9001      # about four turns of the persistent grid (148 x 2 blocks of 8 warps)
+    x = torch.randn(most, H, device="cuda", generator=g)
+    x = x.half() if in_f16 else x
+    res = torch.randn(most, H, device="cuda", generator=g) if with_residual else None
+    gamma = 1 + torch.randn(H, device="cuda", generator=g) * 0.1
+    beta = torch.randn(H, device="cuda", generator=g) * 0.1
+
+    def run(rows):
+        out = torch.full((rows + 1, H), float("nan"), device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+        out32 = torch.full((rows + 1, H), float("nan"), device="cuda")
+        assert pybert.k_layernorm(out_f16, in_f16, x.data_ptr(), None if res is None else res.data_ptr(), gamma.data_ptr(),
+                                  beta.data_ptr(), out.data_ptr(), out32.data_ptr(), rows, H) == 0
+        assert torch.isnan(out[rows].float()).all() and torch.isnan(out32[rows]).all()
+        return out[:rows], out32[:rows]
+
+    few, few32 = run(4096)
+    ref = bert_oracle.layer_norm(x.float() + (0 if res is None else res), gamma, beta)
+    for rows in (4097, 5000, most):
+        out, out32 = run(rows)
+        # fp16: half a step, 2^-12 relative, of values up to 8; fp32: as for the few rows above
+        assert (out.float() - ref[:rows]).abs().max().item() <= (4e-3 if out_f16 else 2e-5)
+        assert (out32 - ref[:rows]).abs().max().item() <= 2e-5
+        assert torch.equal(out[:4096], few) and torch.equal(out32[:4096], few32)

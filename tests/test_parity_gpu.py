@@ -173,6 +173,24 @@ def test_full_size_properties(models, cfg, wname, precision):
     assert bert_oracle.rel_err(full[:2], ref) <= BF16_REL
 
 
+@pytest.mark.parametrize("batch,seq,dist", [(8, 128, "uniform:32:128"), (24, 101, "full"), (70, 64, "full"),
+                                            (47, 100, "uniform:20:100")])
+def test_fp32_rows_do_not_depend_on_the_batch(models, batch, seq, dist):
+    """fp32 passes on both sides of what goes by their size: the GEMMs' ring depth (1.5 CTAs per SM), the
+    LayerNorm kernel and dependent launch (4096 token slots).  The first rows agree with the CPU oracle, and on their
+    own, and in repeated passes, they have the same bits."""
+    m = models("base_affine", "fp32")
+    ids, seg, mask = synth.make_inputs(batch + seq, batch, seq, dist)
+    full = m.encode([ids, seg, mask])
+    for _ in range(3):
+        assert np.array_equal(m.encode([ids, seg, mask]), full)
+    assert np.array_equal(m.encode([ids[:3], seg[:3], mask[:3]]), full[:3])
+    dims = synth.model_dims(False)
+    _, ref = bert_oracle.bert_forward(cases.get_weights("base_affine"), ids[:2], seg[:2], mask[:2], dims["heads"],
+                                      dims["layers"])
+    assert np.abs(full[:2] - ref).max() <= FP32_MAXABS
+
+
 @pytest.mark.parametrize("batch,seq", [(21, 97), (22, 96), (32, 128), (41, 100)])
 def test_fp8_weights_widened_before_the_gemm_keep_every_bit(models, batch, seq):
     """FP8 passes of 2048 token slots and more widen each weight matrix into one scratch matrix just before its GEMM;

@@ -15,6 +15,9 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 BASE_CASES = ["c0_affine", "c2_small", "edge_s17", "edge_b1s1", "edge_nomask", "edge_zero_row", "edge_holes"]
 LARGE_CASES = ["c1_small", "c3_small", "c4_small"]
+# 70 x 64 = 4480 token slots, beyond the 4096 up to which LayerNorm takes a warp per row and launches are dependent;
+# the golden cases have at most 2048.  Seeded inputs, no golden output.
+MANY_ROWS = "rows_70x64"
 SWITCHES = ("CUDABERT_PACK", "CUDABERT_GRAPH", "CUDABERT_PDL", "CUDABERT_LAST_LAYER", "CUDABERT_ATTENTION",
             "CUDABERT_GEMM_PAIR", "CUDABERT_GEMM_SMALL_TILES", "CUDABERT_PRECISION", "CUDABERT_LN",
             "CUDABERT_FP8_OPERAND", "CUDABERT_ATTENTION_TILES", "CUDABERT_FP32_GEMM", "CUDABERT_LN_FOLD", "SWITCH_CHILD_PRECISION")
@@ -22,7 +25,7 @@ SWITCHES = ("CUDABERT_PACK", "CUDABERT_GRAPH", "CUDABERT_PDL", "CUDABERT_LAST_LA
 
 @pytest.fixture(scope="module")
 def run_with(weight_dirs, tmp_path_factory):
-    specs = ["%s:0:%s" % (weight_dirs("base_affine"), ",".join(BASE_CASES)),
+    specs = ["%s:0:%s" % (weight_dirs("base_affine"), ",".join(BASE_CASES + [MANY_ROWS])),
              "%s:1:%s" % (weight_dirs("large_affine"), ",".join(LARGE_CASES))]
     folder = tmp_path_factory.mktemp("switches")
     cache = {}
@@ -51,12 +54,22 @@ def test_scheduling_switches_keep_every_bit(run_with, switch):
     default = run_with()
     name, value = switch.split("=")
     other = run_with(**{name: value})
-    for case in BASE_CASES + LARGE_CASES:
+    for case in BASE_CASES + LARGE_CASES + [MANY_ROWS]:
+        np.testing.assert_array_equal(other[case], default[case], err_msg="%s, case %s" % (switch, case))
+
+
+@pytest.mark.parametrize("switch", ["CUDABERT_PACK=0", "CUDABERT_PDL=1", "CUDABERT_LN=block"])
+def test_scheduling_switches_keep_every_bit_in_fp32(run_with, switch):
+    """The same in fp32 mode, where every producer also writes the bf16 planes that the next GEMM reads."""
+    default = run_with(SWITCH_CHILD_PRECISION="fp32")
+    name, value = switch.split("=")
+    other = run_with(SWITCH_CHILD_PRECISION="fp32", **{name: value})
+    for case in BASE_CASES + LARGE_CASES + [MANY_ROWS]:
         np.testing.assert_array_equal(other[case], default[case], err_msg="%s, case %s" % (switch, case))
 
 
 @pytest.mark.parametrize("switch", ["CUDABERT_ATTENTION=tc", "CUDABERT_ATTENTION=persist", "CUDABERT_ATTENTION=mma",
-                                    "CUDABERT_GEMM_PAIR=0", "CUDABERT_GEMM_SMALL_TILES=1", "CUDABERT_LN_FOLD=1"])
+                                    "CUDABERT_GEMM_PAIR=0", "CUDABERT_LN_FOLD=1"])
 def test_kernel_choice_switches_stay_close(run_with, switch):
     """Another attention kernel or GEMM tile shape rounds at other places, and twelve or twenty-four
     layers of bf16 activations amplify that: the output stays within the bf16 mode's budget against the
