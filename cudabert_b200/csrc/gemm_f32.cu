@@ -133,6 +133,7 @@ gemm_f32_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
 constexpr int PN = 16, PB = 8, PSLICES = 16;
 constexpr int WPITCH = PN + 4;  // the two slices of a warp read weight rows 4 apart: 16 banks apart
 constexpr int POOL_GROUPS = 2;  // 64 column slabs x 2 = 128 CTAs of 152 KB at H = 1024
+constexpr int POOL_TILE_MIN_SEQS = 192;  // see pooler_f32
 
 __global__ void __launch_bounds__(PN * PSLICES)
 pooler_f32_kernel(const float* __restrict__ x, int rows_per_seq, const int* __restrict__ row_start,
@@ -200,24 +201,131 @@ pooler_f32_kernel(const float* __restrict__ x, int rows_per_seq, const int* __re
   }
 }
 
+// The same for many sequences: a CTA takes 32 of them and 64 columns, a thread 4 x 4 outputs, so that two 16-byte reads of
+// shared memory feed 16 multiply-adds and the product is bound by those.  The terms are added in the order of
+// pooler_f32_kernel, so a row has the same bits from either: the loop runs slice after slice (k = 64 j + 4 s .. + 3 for
+// s = 0 .. 15), each slice's sum is finished in registers and added to bias + the sums before.  Slices are copied
+// asynchronously into two buffers, the first one's weights ahead of griddep_wait.
+constexpr int PTM = 32, PTN = 64, PTHREADS = (PTM / 4) * (PTN / 4);
+
+__global__ void __launch_bounds__(PTHREADS)
+pooler_f32_tile_kernel(const float* __restrict__ x, int rows_per_seq, const int* __restrict__ row_start,
+                       const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out, int B, int H) {
+  extern __shared__ float pool_smem[];
+  __shared__ int srow[PTM];               // row of x of the CTA's sequences, -1 beyond the batch
+  const int KS = H / PSLICES, XP = KS + 4;  // a slice's terms; pitch of its inputs: a warp's two rows are 16 banks apart
+  float* xs = pool_smem;                 // [2][PTM][XP]
+  float* ws = xs + 2 * PTM * XP;          // [2][KS][PTN]
+  const int tid = threadIdx.x;
+  const int n0 = blockIdx.x * PTN, b0 = blockIdx.y * PTM;
+  const int c = (tid % (PTN / 4)) * 4, r0 = (tid / (PTN / 4)) * 4;
+  auto load_w = [&](int buf, int s) {
+    for (int i = tid; i < KS * (PTN / 4); i += PTHREADS) {
+      const int kk = i / (PTN / 4), c4 = (i % (PTN / 4)) * 4, k = (kk >> 2) * (4 * PSLICES) + 4 * s + (kk & 3);
+      cp_async16(smem_u32(ws + (buf * KS + kk) * PTN + c4), W + static_cast<size_t>(k) * H + n0 + c4, true);
+    }
+  };
+  auto load_x = [&](int buf, int s) {
+    for (int i = tid; i < PTM * (KS / 4); i += PTHREADS) {
+      const int r = i / (KS / 4), j = i - r * (KS / 4), row = srow[r];
+      const float* src = row < 0 ? x : x + static_cast<size_t>(row) * H + j * (4 * PSLICES) + 4 * s;
+      cp_async16(smem_u32(xs + (buf * PTM + r) * XP + 4 * j), src, row >= 0);
+    }
+  };
+  load_w(0, 0);
+  float v[4][4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float bv = __ldg(bias + n0 + c + q);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r][q] = bv;
+  }
+  griddep_wait();
+  griddep_launch();
+  if (tid < PTM) {
+    const int bb = b0 + tid;
+    srow[tid] = bb >= B ? -1 : row_start ? __ldg(row_start + bb) : bb * rows_per_seq;
+  }
+  __syncthreads();
+  load_x(0, 0);
+  cp_async_commit();
+  for (int s = 0; s < PSLICES; ++s) {
+    const int buf = s & 1;
+    if (s + 1 < PSLICES) {
+      load_w(buf ^ 1, s + 1);
+      load_x(buf ^ 1, s + 1);
+    }
+    cp_async_commit();
+    cp_async_wait<1>();  // all but the slice just requested
+    __syncthreads();
+    const float* xb = xs + (buf * PTM + r0) * XP;
+    const float* wb = ws + buf * KS * PTN + c;
+    float acc[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[r][q] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < KS; k += 4) {
+      float4 xv[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) xv[r] = *reinterpret_cast<const float4*>(xb + r * XP + k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(wb + (k + i) * PTN);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float a = i == 0 ? xv[r].x : i == 1 ? xv[r].y : i == 2 ? xv[r].z : xv[r].w;
+          acc[r][0] = fmaf(a, w.x, acc[r][0]);
+          acc[r][1] = fmaf(a, w.y, acc[r][1]);
+          acc[r][2] = fmaf(a, w.z, acc[r][2]);
+          acc[r][3] = fmaf(a, w.w, acc[r][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[r][q] += acc[r][q];
+    __syncthreads();  // the buffer is free for the slice after next
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    if (b0 + r0 + r < B)
+      *reinterpret_cast<float4*>(out + static_cast<size_t>(b0 + r0 + r) * H + n0 + c) =
+          make_float4(tanhf(v[r][0]), tanhf(v[r][1]), tanhf(v[r][2]), tanhf(v[r][3]));
+}
+
 }  // namespace
 
 int pooler_f32(const float* x, int rows_per_seq, const int* row_start, const float* W, const float* bias, float* out,
                int B, int H, cudaStream_t stream) {
   if (B <= 0 || H <= 0 || (H % 64) != 0 || H > 1024) return -1;
-  // one CTA fits on an SM: beyond POOL_GROUPS groups of sequences a CTA takes several
-  const int groups = (B + PB - 1) / PB;
-  dim3 grid(H / PN, groups < POOL_GROUPS ? groups : POOL_GROUPS);
-  const size_t smem = (static_cast<size_t>(H) * (WPITCH + 2 * PB) + PSLICES * PB * PN) * sizeof(float);
   static std::atomic<bool> attr_set[64] = {};  // per device; a repeated set by a racing thread is harmless
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
     if (cudaFuncSetAttribute(pooler_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (1024 * (WPITCH + 2 * PB) + PSLICES * PB * PN) * static_cast<int>(sizeof(float))) != cudaSuccess)
+                             (1024 * (WPITCH + 2 * PB) + PSLICES * PB * PN) * static_cast<int>(sizeof(float))) != cudaSuccess ||
+        cudaFuncSetAttribute(pooler_f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             2 * (PTM * (1024 / PSLICES + 4) + 1024 / PSLICES * PTN) * static_cast<int>(sizeof(float))) != cudaSuccess)
       return -2;
     if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
   }
+  // The slab kernel's 96 (H = 768) or 128 CTAs take their groups of eight sequences one after the other, some 2.5 us each; a tile's time does not grow until the tiles fill the SMs.  Same bits.  Slab / tiles, us (events around the
+  // launch): H = 768 128 sequences 25 / 33, 192 35 / 33, 256 44 / 33, 1024 154 / 55, 4096 596 / 168; H = 1024 128 30 / 38,
+  // 192 41 / 39, 256 52 / 39, 1024 187 / 82, 4096 729 / 281.
+  if (B >= POOL_TILE_MIN_SEQS) {
+    const dim3 grid(H / PTN, (B + PTM - 1) / PTM);
+    if (grid.y > 65535) return -1;
+    const size_t smem = 2 * (static_cast<size_t>(PTM) * (H / PSLICES + 4) + static_cast<size_t>(H) / PSLICES * PTN) * sizeof(float);
+    return launch_pdl(pooler_f32_tile_kernel, grid, dim3(PTHREADS), smem, stream, x, rows_per_seq, row_start, W, bias, out,
+                      B, H) == cudaSuccess ? 1 : -3;
+  }
+  // one CTA fits on an SM: beyond POOL_GROUPS groups of sequences a CTA takes several
+  const int groups = (B + PB - 1) / PB;
+  dim3 grid(H / PN, groups < POOL_GROUPS ? groups : POOL_GROUPS);
+  const size_t smem = (static_cast<size_t>(H) * (WPITCH + 2 * PB) + PSLICES * PB * PN) * sizeof(float);
   return launch_pdl(pooler_f32_kernel, grid, dim3(PN * PSLICES), smem, stream, x, rows_per_seq, row_start, W, bias, out,
                     B, H) == cudaSuccess ? 1 : -3;
 }

@@ -206,6 +206,35 @@ def test_fp8_weights_widened_before_the_gemm_keep_every_bit(models, batch, seq):
     assert np.array_equal(m.encode([ids[:2], seg[:2], mask[:2]]), full[:2])
 
 
+@pytest.mark.parametrize("wname", ["base_affine", "large_affine"])
+def test_pooler_of_few_and_of_many_sequences(models, wname):
+    """Up to 191 sequences the pooler keeps slabs of its weights in shared memory, from 192 on it works in tiles of 32
+    sequences and 64 columns.  At the edges of both: the first rows have the bits they have alone, and
+    every row is tanh(h W + b) of the hidden state of its first token, evaluated in float64 (a dot
+    product of at most 1024 fp32 terms of order 0.1: rounding below 1024 * 2^-24 of their sum)."""
+    from cudabert_b200.cuda_bert import pybert
+    m = models(wname, "bf16")
+    H = m.hidden_size
+    w = cases.get_weights(wname)
+    kernel, bias = (w[k].astype(np.float64) for k in ("bert_pooler_dense_kernel", "bert_pooler_dense_bias"))
+    S, most = 5, 1057
+    ids, seg, mask = synth.make_inputs(11, most, S, "uniform:1:%d" % S)
+    alone = np.concatenate([m.encode([ids[i:i + 61], seg[i:i + 61], mask[i:i + 61]]) for i in range(0, most, 61)])
+    for B in (1, 8, 9, 190, 191, 192, 193, 223, 224, 225, 1024, most):
+        part = [ids[:B], seg[:B], mask[:B]]
+        got = m.encode(part)
+        assert np.array_equal(got, alone[:B]), "B = %d" % B
+        ret = pybert.inference(m.model, part[0], part[1], B, S, part[2])
+        pybert.check(m.model)
+        hidden, pooled = np.empty((B, S, H), np.float32), np.empty((B, H), np.float32)
+        assert pybert.copy_to_host(hidden.ctypes.data, ret.tensor, hidden.nbytes) == 0
+        assert pybert.copy_to_host(pooled.ctypes.data, ret.Pooled_Output, pooled.nbytes) == 0
+        assert np.array_equal(pooled, got), "B = %d" % B
+        first = hidden[:, 0].astype(np.float64)
+        bound = 1e-6 + 2.0 ** -14 * (np.abs(first) @ np.abs(kernel))
+        assert (np.abs(pooled - np.tanh(first @ kernel + bias)) <= bound).all(), "B = %d" % B
+
+
 @pytest.mark.parametrize("precision", ["bf16", "fp8", "fp32"])
 def test_weight_cache_gives_the_same_model(weight_dirs, tmp_path, monkeypatch, precision):
     """CUDABERT_WEIGHT_CACHE: the first load writes the device-ready weights as one file, the second
