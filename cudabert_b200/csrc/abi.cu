@@ -316,7 +316,7 @@ int cudabert_k_gemm_f32_tensor(const float* A_dev, int lda, const float* W_dev, 
     rc = 2;
   CUtensorMap tmA, tmW;
   if (!rc && (!cb::make_tmap_16bit_kmajor(&tmA, a3, M, 3ull * K, 6ull * K, 128) ||
-              !cb::make_tmap_16bit_kmajor(&tmW, w3, N, 3ull * K, 6ull * K, cb::gemm_split_w_box_rows(N))))
+              !cb::make_tmap_16bit_kmajor(&tmW, w3, N, 3ull * K, 6ull * K, cb::SPLIT_W_BOX_ROWS)))
     rc = 2;
   if (!rc) {
     cudaMemset(err, 0, sizeof(int));

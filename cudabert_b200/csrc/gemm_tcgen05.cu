@@ -7,11 +7,12 @@
 // `cuApplyLayerNorm` does in place (ops/layernorm.cu:152-158) and the pooler's tanh
 // (ops/elementwise.cu:57-70).
 //
-// Two variants share the epilogue.  `gemm_tcgen05_pair_kernel` (default when N is a multiple of
+// Three variants share the epilogue.  `gemm_tcgen05_pair_kernel` (default when N is a multiple of
 // 256) runs CTA pairs: a 256 x 256 tile per pair, `tcgen05.mma.cta_group::2`, each CTA loading its
 // own 128 rows of A and its own half (128 rows) of the W tile, so an SM fills 32 KB of shared
-// memory per k-block instead of 48 KB; the operand feed is what bounds the single-CTA variant.
-// Loads are never shared between CTAs.  `gemm_tcgen05_kernel` is the single-CTA variant:
+// memory per k-block instead of 48 KB.  `gemm_tcgen05_thin_kernel` takes products of few rows in narrow
+// single-CTA tiles.  fp32 mode has a kernel and an epilogue of its own, `gemm_split3_kernel`.
+// Loads are never shared between CTAs.  `gemm_tcgen05_kernel` is the single-CTA variant for the other widths:
 //
 // Structure (one persistent CTA per SM, 320 threads):
 //   warp 0, one lane   TMA producer: per k-block one 128x64 tile of A and one BNx64 tile of W
@@ -1090,8 +1091,10 @@ gemm_tcgen05_thin_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 // tensor-core accumulations also round less: against float64 the errors are smaller than of the six-pass loop
 // (tests/test_kernels_gpu.py::test_gemm_f32_on_tensor_cores prints them).
 // Measured per launch inside a BERT-base pass (one B200), against the six-pass loop: 657 rows QKV 29 -> 18 us,
-// attention-output 22 -> 14, FFN1 29 -> 20, FFN2 67 -> 27.  What bounds it is shared-memory bandwidth: 288 KB per slice of
-// 64 columns (192 read by the MMAs, 96 written by TMA) are 2300 clocks at 128 B per clock, the MMAs 1536.
+// attention-output 22 -> 14, FFN1 29 -> 20, FFN2 67 -> 27.  On paper shared memory is the nearest limit: 288 KB per slice
+// of 64 columns (192 read by the MMAs, 96 written by TMA) are 2300 clocks at 128 B per clock, the MMAs 1536.  The
+// counters do not show it as the bound: with cold caches both it and the tensor pipe are 50 - 53 % busy in QKV, FFN1 and FFN2
+// at 657 rows, 29 % in attention-output, the rest being each CTA's start and epilogue in launches of about one turn.
 template <int SLOTS_>
 struct SplitCfg {
   static constexpr int SLOTS = SLOTS_;
@@ -1232,8 +1235,6 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         umma_commit(tfull_bar);
       }
     }
-  } else {
-    griddep_wait();
   }
   __syncwarp();
   griddep_wait();  // every thread: the live row count below is a predecessor's
@@ -1601,8 +1602,6 @@ int wait_timeout_probe(int* err_flag, unsigned long long limit_ns, cudaStream_t 
 }
 
 int gemm_block_n(int N) { return (N % 256 == 0) ? 256 : 128; }
-
-int gemm_split_w_box_rows(int N) { return 128; }
 
 // CUDABERT_GEMM_SMALL_TILES=0 keeps every product on the kernel that large ones take (same bits)
 static bool thin_enabled() {

@@ -21,9 +21,10 @@ namespace cb {
 // pass itself writes go to kernels that read them after the wait); a caller who cannot vouch for that
 // opens a NoPdlScope.  Everything else is read or written after the wait.
 // Whether launch_pdl asks for programmatic dependent launch.  Measured: it shortens a forward pass
-// of a few thousand tokens (BERT-base, 8 x 128: 0.86 against 0.94 ms) and costs about 1 % on one of
-// 25 600 tokens, so the forward pass switches it per call (`tl_pdl_allowed`); CUDABERT_PDL=0 turns it
-// off everywhere, CUDABERT_PDL=1 on for every forward pass, but not inside a NoPdlScope.
+// of up to some 4096 token slots and lengthens one of 8192 and more (us, off / on, S = 128; BERT-base 1024 slots 655 / 593,
+// 4096 1200 / 1123, 6144 1398 / 1388, 8192 1923 / 1947, 16384 3417 / 3472; BERT-large 1483 / 1381, 3060 / 2940,
+// 4498 / 4562, 5470 / 5688, 10526 / 10812), so the forward pass switches it per call (`tl_pdl_allowed`, PDL_MAX_TOKENS);
+// CUDABERT_PDL=0 turns it off everywhere, CUDABERT_PDL=1 on for every forward pass, but not inside a NoPdlScope.
 inline thread_local bool tl_pdl_allowed = true;
 inline thread_local int tl_plain_order = 0;  // NoPdlScopes open on this thread
 inline bool pdl_enabled() {
@@ -164,7 +165,7 @@ int wait_timeout_probe(int* err_flag, unsigned long long limit_ns, cudaStream_t 
 int gemm_w_box_rows(int N);
 bool gemm_uses_pairs(int N);  // the CTA-pair kernel (256 x 256 tiles) serves this width
 // The same for the W operand of an EPI_SPLIT3 GEMM ([N, 3 K] bf16 planes; 128 x 128 tiles).
-int gemm_split_w_box_rows(int N);
+constexpr int SPLIT_W_BOX_ROWS = 128;
 // Encode a 2-D tiled map over a row-major matrix of 16-bit elements [rows, cols] with
 // `row_stride_bytes` between rows, box = 64 columns (128 bytes, 128-byte swizzle) x `box_rows` rows.
 bool make_tmap_16bit_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,

@@ -257,7 +257,7 @@ bool Model::finish_dense(DenseWeight* d, int prec) {
   if (prec == PREC_FP32_SPLIT) {
     if (d->N % 128 != 0 || d->K % 64 != 0) return fail(1, "the tensor-core fp32 GEMM needs widths in multiples of 128 and depths of 64");
     if (!make_tmap_16bit_kmajor(&d->tmap, d->w, d->N, 3 * static_cast<uint64_t>(d->K), static_cast<uint64_t>(d->K) * 6,
-                                gemm_split_w_box_rows(d->N)))
+                                SPLIT_W_BOX_ROWS))
       return fail(2, "cuTensorMapEncodeTiled failed for a weight matrix");
     return true;
   }

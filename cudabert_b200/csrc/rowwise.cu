@@ -153,8 +153,8 @@ __device__ __forceinline__ void load4<__half>(const __half* p, float (&v)[4]) {
 }
 
 // out = LayerNorm(in + residual): `in` is the dense projection's output (fp32, or fp16 from the
-// tensor-core GEMM), `residual` (may be null) the fp32 residual stream.  One row per warp, for launches whose rows
-// all find a warp at once; what bounds it there is the chain of memory latencies, so nothing waits that need
+// tensor-core GEMM), `residual` (may be null) the fp32 residual stream.  One row per warp, for launches of up to
+// LN_FEW_ROWS rows; what bounds it there is the chain of memory latencies, so nothing waits that need
 // not: gamma and beta, which no kernel writes, are requested before griddep_wait, and the row is
 // requested together with the live row count instead of after it (rows beyond it exist in the buffers and are
 // not stored).  Same arithmetic and bits as layernorm_persist_kernel.  Measured on a B200 as the time from
@@ -403,7 +403,7 @@ int embed_layernorm(const int* ids, const int* seg, const float* word, const flo
                     type, gamma, beta, out, out_f32, tokens, S, H, vocab, err_flag, row_start, planes) == cudaSuccess ? 1 : -3;
 }
 
-// Persistent form of layernorm_kernel, the default: a fixed grid (two blocks of eight warps per SM)
+// Persistent form of layernorm_kernel, for more than LN_FEW_ROWS rows: a fixed grid (two blocks of eight warps per SM)
 // whose warps stride over the live rows, so rows that do not exist cost no blocks, and a warp issues
 // the loads of its next row before it reduces and stores the current one, holding them raw
 // (unconverted) so that nothing waits on them until the next turn.  Same arithmetic, same bits as
@@ -498,9 +498,13 @@ int layernorm(const TIn* x, const float* residual, const float* gamma, const flo
               int tokens, int H, const int* rows_dev, cudaStream_t stream, const int* res_rows, int res_stride,
               __nv_bfloat16* planes) {
   if (tokens <= 0 || !ln_shape_ok(H)) return -1;
-  // As long as every row finds a warp at once (148 SMs hold well over 4096 warps) a launch is one row's chain of latencies,
-  // and the one-row-per-warp kernel with its early loads is the faster one: BERT-large 32 x 128 (4096 rows) 3131 -> 3027 us
-  // per pass.  Beyond, rows come in turns and the persistent grid's look-ahead pays (its comment).
+  // Few rows: one row's chain of latencies is most of the launch, and the one-row-per-warp kernel with its early loads is
+  // the faster one.  Its 128 registers (gamma and beta are held in them; 130 with fp32 input) let 2368 (1776) rows be
+  // in flight on 148 SMs, so from there on rows come in turns, and with more turns the persistent grid's look-ahead (its comment)
+  // gains on it.  The line lies where they meet.  Whole passes, S = 128, us, row per warp / persistent: BERT-base 1024 rows
+  // 593 / 625, 2048 740 / 771, 4096 1123 / 1123, 6144 1462 / 1414, 8192 1977 / 1910, 16384 3556 / 3383; BERT-large 1380 / 1480,
+  // 1855 / 1938, 3001 / 3046, 4581 / 4461, 5612 / 5536, 10909 / 10366; BERT-base in fp32 1952 / 2012, 3212 / 3226,
+  // 5326 / 5336, 7532 / 7540, 10154 / 9977, 19421 / 19305.
   if (layernorm_persistent() && tokens > LN_FEW_ROWS) {
     const int warps_per_block = LNP_THREADS / 32;
     const int want = (tokens + warps_per_block - 1) / warps_per_block;
